@@ -26,6 +26,23 @@ constexpr int WARPS = 8;        // warps per block
 constexpr int CPL = 8;          // channels per lane
 constexpr int CPW = 32 * CPL;   // channels per warp
 
+// The 8 channels of a lane are two runs of four, at Chan<T>::off(lane, 0) and (lane, 1) of the warp's 256, T the type
+// that the inner loop loads. BF16: 8 channels side by side, one 16-byte load. float32: channels 4 lane and 128 + 4
+// lane, so that each 16-byte load of the warp covers 512 contiguous bytes; with 8 channels side by side every load
+// touched half of each of 8 lines, and L1 gave 64 instead of 87 or more bytes per clock and SM (measured, L1 hits).
+template <typename T> struct Chan;
+template <> struct Chan<float> {
+    static __device__ __forceinline__ int off(int lane, int h) { return 4 * lane + h * (CPW / 2); }
+};
+template <> struct Chan<__nv_bfloat16> {
+    static __device__ __forceinline__ int off(int lane, int h) { return CPL * lane + 4 * h; }
+};
+
+__device__ __forceinline__ void st4(float *p, const float *r)
+{
+    *reinterpret_cast<float4 *>(p) = make_float4(r[0], r[1], r[2], r[3]);
+}
+
 __device__ __forceinline__ void ld8(const float *p, float4 &a, float4 &b)
 {
     a = __ldg(reinterpret_cast<const float4 *>(p));
@@ -58,6 +75,11 @@ __device__ __forceinline__ void st8(__nv_bfloat16 *p, const float (&r)[CPL])
 {
     *reinterpret_cast<uint4 *>(p) = make_uint4(pack_bf16(r[0], r[1]), pack_bf16(r[2], r[3]), pack_bf16(r[4], r[5]),
                                                pack_bf16(r[6], r[7]));
+}
+
+__device__ __forceinline__ void st4(__nv_bfloat16 *p, const float *r)
+{
+    *reinterpret_cast<uint2 *>(p) = make_uint2(pack_bf16(r[0], r[1]), pack_bf16(r[2], r[3]));
 }
 
 // a += w p on 8 channels: four paired FMAs (FFMA2, sm_100), each lane of a pair rounded once as fmaf does
@@ -185,19 +207,52 @@ __global__ void ray_table_kernel(const float4 *__restrict__ geo, int n_angles, i
     if (!row_ptr) counts[row] = n;
 }
 
+// The lane's runs of the 256 channels from kblk on: k[h] their first channels (outputs: those below kstride), o[h] the
+// offsets its loads use (runs past kb read channel kblk instead, and their sums are dropped).
+template <typename T>
+__device__ __forceinline__ void lane_runs(int lane, int kblk, int kb, int (&k)[2], int (&o)[2])
+{
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        o[h] = Chan<T>::off(lane, h);
+        k[h] = kblk + o[h];
+    }
+    const bool two = sizeof(T) == 4;
+    o[1] = (two ? k[1] : k[0]) < kb ? o[1] : 0;
+    o[0] = k[0] < kb ? o[0] : 0;
+}
+
+// one output row of the warp's channels: scale r on channels below kb, 0 on the padding channels up to kstride
+template <typename ST>
+__device__ __forceinline__ void store_row(ST *row, const int (&k)[2], int kstride, int kb, float scale,
+                                          const float (&r)[CPL])
+{
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        if (k[h] >= kstride) continue;
+        float o[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) o[q] = k[h] + q < kb ? __fmul_rn(scale, r[4 * h + q]) : 0.0f;
+        st4(row + k[h], o);
+    }
+}
+
 // Raw channel loads of the table-driven forward: 8 channels kept as loaded (2 x float4, or 8 BF16 in a uint4) until
 // their FMAs, so that a warp can hold many taps' loads in flight in few registers.
 template <typename IT> struct Raw8;
 template <> struct Raw8<float> { float4 a, b; };
 template <> struct Raw8<__nv_bfloat16> { uint4 u; };
 
-__device__ __forceinline__ void ldraw(const float *p, Raw8<float> &r) { ld8(p, r.a, r.b); }
-__device__ __forceinline__ void ldraw(const __nv_bfloat16 *p, Raw8<__nv_bfloat16> &r)
+// o0, o1: the lane's two runs (Chan), those outside the row moved to channel 0 by lane_runs (their sums are dropped)
+__device__ __forceinline__ void ldraw(const float *p, int o0, int o1, Raw8<float> &r)
 {
-    r.u = __ldg(reinterpret_cast<const uint4 *>(p));
+    r.a = __ldg(reinterpret_cast<const float4 *>(p + o0));
+    r.b = __ldg(reinterpret_cast<const float4 *>(p + o1));
 }
-__device__ __forceinline__ void zraw(Raw8<float> &r) { r.a = r.b = make_float4(0.f, 0.f, 0.f, 0.f); }
-__device__ __forceinline__ void zraw(Raw8<__nv_bfloat16> &r) { r.u = make_uint4(0, 0, 0, 0); }
+__device__ __forceinline__ void ldraw(const __nv_bfloat16 *p, int o0, int, Raw8<__nv_bfloat16> &r)
+{
+    r.u = __ldg(reinterpret_cast<const uint4 *>(p + o0));
+}
 __device__ __forceinline__ void accraw(float (&a)[CPL], float w, const Raw8<float> &r) { acc8(a, w, r.a, r.b); }
 __device__ __forceinline__ void accraw(float (&a)[CPL], float w, const Raw8<__nv_bfloat16> &r)
 {
@@ -206,60 +261,69 @@ __device__ __forceinline__ void accraw(float (&a)[CPL], float w, const Raw8<__nv
 }
 
 // Table-driven forward: warp per (angle, bin, 256 channels), angle a of the launch = angles[a] of the table (angles
-// NULL: a); the same taps, weights and summation order as radon_forward_v4, so the same bits. U taps are loaded
-// before their FMAs (16 for a BF16 image: 0.32 -> 0.28 ms per ti256 launch of 18 angles x 1012 channels).
+// NULL: a); the same taps, weights and summation order as radon_forward_v4, so the same bits. Bound by the L1 data
+// path and L2 (a float32 launch of all 360 angles at 256 x 256 pixels, 1012 channels: 85 % and 80 % of their peaks);
+// what it needs is loads in flight at few registers: a software pipeline over groups of U taps, 2 of a float32 image
+// (60 registers; without it ptxas kept 40 and one tap's loads in flight) and 4 of a BF16 one. That launch went from 10.9
+// to 7.2 ms, 18 angles from 0.68 to 0.44 ms (U = 4: 8.1 and 0.46, U = 8: 11.7 and 0.64).
 template <typename ST, typename IT>
 __global__ void __launch_bounds__(32 * WARPS) radon_forward_table(
     const IT *__restrict__ img, ST *__restrict__ sino, int64_t sld, const int32_t *__restrict__ row_ptr,
     const int2 *__restrict__ entries, const int32_t *__restrict__ angles, int ns, int kstride, int kb, float scale)
 {
-    constexpr int U = sizeof(IT) == 2 ? 16 : 8;   // taps in flight: 16 x 16 bytes (BF16), 8 x 32 bytes (float32)
+    constexpr int U = sizeof(IT) == 2 ? 4 : 2;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int s = blockIdx.x * WARPS + warp;
     const int al = blockIdx.y;
-    const int k = blockIdx.z * CPW + lane * CPL;
+    const int kblk = blockIdx.z * CPW;
     if (s >= ns) return;
-    const bool live = k < kstride;
-    ST *out = sino + ((int64_t)al * ns + s) * sld + k;
-    if (blockIdx.z * CPW >= kb) {
-        const float zero[CPL] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        if (live) st8(out, zero);
-        return;
-    }
-    const bool load = k < kb;
-    const int a = angles ? __ldg(angles + al) : al;
-    const int64_t r = (int64_t)a * ns + s;
-    int e = __ldg(row_ptr + r);
-    const int e1 = __ldg(row_ptr + r + 1);
-    const IT *base = img + (load ? k : 0);
+    int k[2], o[2];
+    lane_runs<IT>(lane, kblk, kb, k, o);
+    ST *out = sino + ((int64_t)al * ns + s) * sld;
     float acc[CPL];
 #pragma unroll
     for (int c = 0; c < CPL; ++c) acc[c] = 0.0f;
-    for (; e + U <= e1; e += U) {
-        int2 t[U];
-        Raw8<IT> q[U];
+    if (kblk < kb) {                                       // not padding channels only
+        const int a = angles ? __ldg(angles + al) : al;
+        const int64_t r = (int64_t)a * ns + s;
+        int e = __ldg(row_ptr + r);
+        const int e1 = __ldg(row_ptr + r + 1);
+        const IT *base = img + kblk;
+        // software pipeline over groups of U taps: the next group's pixels are loaded while this one's FMAs run
+        if (e + U <= e1) {
+            int2 t[U], tn[U];
+            Raw8<IT> q[U];
 #pragma unroll
-        for (int i = 0; i < U; ++i) t[i] = __ldg(entries + e + i);
+            for (int i = 0; i < U; ++i) t[i] = __ldg(entries + e + i);
 #pragma unroll
-        for (int i = 0; i < U; ++i) {
-            zraw(q[i]);
-            if (load) ldraw(base + (int64_t)t[i].x * kstride, q[i]);
+            for (int i = 0; i < U; ++i) ldraw(base + (int64_t)t[i].x * kstride, o[0], o[1], q[i]);
+            e += U;
+#pragma unroll 2
+            for (; e + U <= e1; e += U) {
+                Raw8<IT> qn[U];
+#pragma unroll
+                for (int i = 0; i < U; ++i) tn[i] = __ldg(entries + e + i);
+#pragma unroll
+                for (int i = 0; i < U; ++i) ldraw(base + (int64_t)tn[i].x * kstride, o[0], o[1], qn[i]);
+#pragma unroll
+                for (int i = 0; i < U; ++i) accraw(acc, __int_as_float(t[i].y), q[i]);
+#pragma unroll
+                for (int i = 0; i < U; ++i) {
+                    t[i] = tn[i];
+                    q[i] = qn[i];
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < U; ++i) accraw(acc, __int_as_float(t[i].y), q[i]);
         }
-#pragma unroll
-        for (int i = 0; i < U; ++i) accraw(acc, __int_as_float(t[i].y), q[i]);
+        for (; e < e1; ++e) {
+            const int2 t = __ldg(entries + e);
+            Raw8<IT> q;
+            ldraw(base + (int64_t)t.x * kstride, o[0], o[1], q);
+            accraw(acc, __int_as_float(t.y), q);
+        }
     }
-    for (; e < e1; ++e) {
-        const int2 t = __ldg(entries + e);
-        Raw8<IT> q;
-        zraw(q);
-        if (load) ldraw(base + (int64_t)t.x * kstride, q);
-        accraw(acc, __int_as_float(t.y), q);
-    }
-    if (!live) return;
-    float o[CPL];
-#pragma unroll
-    for (int q = 0; q < CPL; ++q) o[q] = (k + q < kb) ? __fmul_rn(scale, acc[q]) : 0.0f;
-    st8(out, o);
+    store_row(out, k, kstride, kb, scale, acc);
 }
 
 // ------------------------------------------------------------------------------------------------ grouped table
@@ -327,83 +391,76 @@ __global__ void ray_gtable_kernel(const float4 *__restrict__ geo, int n_angles, 
     if (!row_ptr) counts[row] = n;
 }
 
-// Grouped-table forward (float32 image and sinogram rows): warp per (angle, GB bins, 256 channels); U pixels in
-// flight, each pixel's FMAs into the bins whose weight is not 0 (a branch the whole warp takes).
+// Grouped-table forward of a float32 image: warp per (angle, GB bins, 256 channels); U pixels in flight, each pixel's
+// FMAs into the bins whose weight is not 0 (a branch the whole warp takes). A block's warps take GA consecutive angles
+// of two groups: the rays of neighbouring angles through the same bins cross nearly the same pixels, so the block
+// finds them in L1 (hit rate 10 -> 70 %, L2 throughput 59 -> 23 % of its peak), which leaves the L1 data path as
+// its bound (76 %). 360 angles at 256 x 256 pixels, 1012 channels: 10.2 ms with a lane's 8 channels side by side, 7.6
+// with whole 512-byte loads (Chan), 6.6 with the block over angles (8 angles of one group: 6.7).
+constexpr int GA = 4;           // angles per block
+
+template <typename ST>
 __global__ void __launch_bounds__(32 * WARPS) radon_forward_gtable(
-    const float *__restrict__ img, float *__restrict__ sino, const int32_t *__restrict__ row_ptr,
-    const int32_t *__restrict__ pix, const float4 *__restrict__ wts, const int32_t *__restrict__ angles, int ns,
-    int kstride, int kb, float scale)
+    const float *__restrict__ img, ST *__restrict__ sino, int64_t sld, const int32_t *__restrict__ row_ptr,
+    const int32_t *__restrict__ pix, const float4 *__restrict__ wts, const int32_t *__restrict__ angles, int n_angles,
+    int ns, int kstride, int kb, float scale)
 {
     constexpr int U = 4;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int ng = (ns + GB - 1) / GB;
-    const int grp = blockIdx.x * WARPS + warp;
-    const int al = blockIdx.y;
-    const int k = blockIdx.z * CPW + lane * CPL;
-    if (grp >= ng) return;
-    const bool live = k < kstride;
+    const int grp = blockIdx.x * (WARPS / GA) + warp / GA;
+    const int al = blockIdx.y * GA + warp % GA;
+    const int kblk = blockIdx.z * CPW;
+    if (grp >= ng || al >= n_angles) return;
+    int k[2], o[2];
+    lane_runs<float>(lane, kblk, kb, k, o);
     const int s0 = grp * GB;
-    float *out = sino + ((int64_t)al * ns + s0) * kstride + k;
+    ST *out = sino + ((int64_t)al * ns + s0) * sld;
     const int nb = min(GB, ns - s0);
-    if (blockIdx.z * CPW >= kb) {
-        const float zero[CPL] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        if (live)
-            for (int j = 0; j < nb; ++j) st8(out + (int64_t)j * kstride, zero);
-        return;
-    }
-    const bool load = k < kb;
-    const int a = angles ? __ldg(angles + al) : al;
-    const int64_t r = (int64_t)a * ng + grp;
-    int e = __ldg(row_ptr + r);
-    const int e1 = __ldg(row_ptr + r + 1);
-    const float *base = img + (load ? k : 0);
     float acc[GB][CPL];
 #pragma unroll
     for (int j = 0; j < GB; ++j)
 #pragma unroll
         for (int c = 0; c < CPL; ++c) acc[j][c] = 0.0f;
-    for (; e + U <= e1; e += U) {
-        int p[U];
-        float4 w[U];
-        Raw8<float> q[U];
+    if (kblk < kb) {                                       // not padding channels only
+        const int a = angles ? __ldg(angles + al) : al;
+        const int64_t r = (int64_t)a * ng + grp;
+        int e = __ldg(row_ptr + r);
+        const int e1 = __ldg(row_ptr + r + 1);
+        const float *base = img + kblk;
+        for (; e + U <= e1; e += U) {
+            int p[U];
+            float4 w[U];
+            Raw8<float> q[U];
 #pragma unroll
-        for (int i = 0; i < U; ++i) {
-            p[i] = __ldg(pix + e + i);
-            w[i] = __ldg(wts + e + i);
+            for (int i = 0; i < U; ++i) {
+                p[i] = __ldg(pix + e + i);
+                w[i] = __ldg(wts + e + i);
+            }
+#pragma unroll
+            for (int i = 0; i < U; ++i) ldraw(base + (int64_t)p[i] * kstride, o[0], o[1], q[i]);
+#pragma unroll
+            for (int i = 0; i < U; ++i) {
+                if (w[i].x != 0.0f) accraw(acc[0], w[i].x, q[i]);
+                if (w[i].y != 0.0f) accraw(acc[1], w[i].y, q[i]);
+                if (w[i].z != 0.0f) accraw(acc[2], w[i].z, q[i]);
+                if (w[i].w != 0.0f) accraw(acc[3], w[i].w, q[i]);
+            }
         }
-#pragma unroll
-        for (int i = 0; i < U; ++i) {
-            zraw(q[i]);
-            if (load) ldraw(base + (int64_t)p[i] * kstride, q[i]);
-        }
-#pragma unroll
-        for (int i = 0; i < U; ++i) {
-            if (w[i].x != 0.0f) accraw(acc[0], w[i].x, q[i]);
-            if (w[i].y != 0.0f) accraw(acc[1], w[i].y, q[i]);
-            if (w[i].z != 0.0f) accraw(acc[2], w[i].z, q[i]);
-            if (w[i].w != 0.0f) accraw(acc[3], w[i].w, q[i]);
+        for (; e < e1; ++e) {
+            const int p = __ldg(pix + e);
+            const float4 w = __ldg(wts + e);
+            Raw8<float> q;
+            ldraw(base + (int64_t)p * kstride, o[0], o[1], q);
+            if (w.x != 0.0f) accraw(acc[0], w.x, q);
+            if (w.y != 0.0f) accraw(acc[1], w.y, q);
+            if (w.z != 0.0f) accraw(acc[2], w.z, q);
+            if (w.w != 0.0f) accraw(acc[3], w.w, q);
         }
     }
-    for (; e < e1; ++e) {
-        const int p = __ldg(pix + e);
-        const float4 w = __ldg(wts + e);
-        Raw8<float> q;
-        zraw(q);
-        if (load) ldraw(base + (int64_t)p * kstride, q);
-        if (w.x != 0.0f) accraw(acc[0], w.x, q);
-        if (w.y != 0.0f) accraw(acc[1], w.y, q);
-        if (w.z != 0.0f) accraw(acc[2], w.z, q);
-        if (w.w != 0.0f) accraw(acc[3], w.w, q);
-    }
-    if (!live) return;
 #pragma unroll
-    for (int j = 0; j < GB; ++j) {
-        if (j >= nb) break;
-        float o[CPL];
-#pragma unroll
-        for (int q = 0; q < CPL; ++q) o[q] = (k + q < kb) ? __fmul_rn(scale, acc[j][q]) : 0.0f;
-        st8(out + (int64_t)j * kstride, o);
-    }
+    for (int j = 0; j < GB; ++j)
+        if (j < nb) store_row(out + (int64_t)j * sld, k, kstride, kb, scale, acc[j]);
 }
 
 // ------------------------------------------------------------------------------------------------ backward
@@ -416,12 +473,48 @@ __device__ __forceinline__ void primal_step(float &x, float &z, float t, float d
     x = t > 0.0f ? fmaxf(0.0f, __fsub_rn(x, __fmul_rn(t, __fadd_rn(zb, lam)))) : 0.0f;
 }
 
-// MODE 0: img (npix, kstride) = backprojection; MODE 1: the backprojection dz is applied to x, z (T the steps):
-// z += dz; x = T > 0 ? max(0, x - T (z + inv_p dz + lam)) : 0. plist (MODE 0, optional): only the pixels plist[0 ..
-// n_out-1], output row r for pixel plist[r] (the same arithmetic per pixel as the whole image).
-// P channel groups of 256 per warp (lane: channels k, k + 256, ...): the pixel's taps and weights are computed once for
-// P x 8 channels per lane, which halves the geometry work per FMA at P = 2; every channel sums the same terms in the
-// same order whatever P is.
+// A pixel's result on the lane's run h of four channels from k on: MODE 0 writes the backprojection acc to img, MODE 1
+// applies it to x (img), z with the steps T and writes the BF16 copy of x. Channels kb .. kstride-1 are padding: MODE 0
+// writes 0, MODE 1 takes dz = 0 (which leaves z, and x, 0 there, unchanged); a warp with padding channels only does
+// not touch MODE 1's arrays.
+template <int MODE>
+__device__ __forceinline__ void finish_run(float *img, float *z, const float *T, __nv_bfloat16 *xb, int64_t row, int k,
+                                           int kstride, int kb, const float *acc, float inv_p, float lam)
+{
+    if (k >= kstride) return;
+    const int64_t o = row * kstride + k;
+    float r[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) r[c] = k + c < kb ? acc[c] : 0.0f;
+    if (MODE == 0) {
+        st4(img + o, r);
+        return;
+    }
+    float4 *xp = reinterpret_cast<float4 *>(img + o), *zp = reinterpret_cast<float4 *>(z + o);
+    float4 xv = *xp, zv = *zp;
+    const float4 tv = __ldg(reinterpret_cast<const float4 *>(T + o));
+    primal_step(xv.x, zv.x, tv.x, r[0], inv_p, lam);
+    primal_step(xv.y, zv.y, tv.y, r[1], inv_p, lam);
+    primal_step(xv.z, zv.z, tv.z, r[2], inv_p, lam);
+    primal_step(xv.w, zv.w, tv.w, r[3], inv_p, lam);
+    *xp = xv;
+    *zp = zv;
+    const float xn[4] = {xv.x, xv.y, xv.z, xv.w};
+    if (xb) st4(xb + o, xn);           // the BF16 copy of x the next forward projection reads
+}
+
+// 8 channels of a sinogram row in float32: the lane's two runs (o0, o1 as lane_runs gives them)
+__device__ __forceinline__ void ldrow(const float *p, int o0, int o1, float4 &a, float4 &b)
+{
+    a = __ldg(reinterpret_cast<const float4 *>(p + o0));
+    b = __ldg(reinterpret_cast<const float4 *>(p + o1));
+}
+__device__ __forceinline__ void ldrow(const __nv_bfloat16 *p, int o0, int, float4 &a, float4 &b) { ld8(p + o0, a, b); }
+
+// Any tap count and any pixels: img (npix, kstride) = backprojection; plist (optional): only the pixels plist[0 ..
+// n_out-1], output row r for pixel plist[r] (the same arithmetic per pixel as the whole image). MODE as finish_run.
+// P channel groups of 256 per warp: the pixel's taps and weights are computed once for P x 8 channels per lane; every
+// channel sums the same terms in the same order whatever P is.
 template <int KERNEL, int MODE, typename ST, int P>
 __global__ void __launch_bounds__(32 * WARPS) radon_backward_v3(
     const ST *__restrict__ sino, int64_t sld, float *__restrict__ img, const float4 *__restrict__ geo, int n_angles, int nx,
@@ -434,24 +527,15 @@ __global__ void __launch_bounds__(32 * WARPS) radon_backward_v3(
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t p = (int64_t)blockIdx.x * WARPS + warp;     // output row
     const int kblk = blockIdx.y * CPW * P;
-    if (p >= n_out || kblk + lane * CPL >= kstride) return;
-    // group h: channels kblk + h CPW + lane CPL (+0..7); live: inside kstride; data: not a block of padding only
-    bool live[P], data[P];
+    if (p >= n_out) return;
+    int k[P][2], o[P][2];
+    bool data[P];                          // not a group of padding channels only
 #pragma unroll
     for (int h = 0; h < P; ++h) {
-        live[h] = kblk + h * CPW + lane * CPL < kstride;
-        data[h] = live[h] && kblk + h * CPW < kb;
+        lane_runs<ST>(lane, kblk + h * CPW, kb, k[h], o[h]);
+        data[h] = kblk + h * CPW < kb;
     }
     const int64_t pix = plist ? (int64_t)__ldg(plist + p) : p;
-    if (!data[0]) {                        // padding channels only: the backprojection is 0 there
-        if (MODE == 0) {
-            const float zero[CPL] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-            for (int h = 0; h < P; ++h)
-                if (live[h]) st8(img + p * kstride + kblk + h * CPW + lane * CPL, zero);
-        }
-        return;                            // MODE 1: dz = 0 leaves z, and x (0 on padding channels), unchanged
-    }
     const int px = (int)(pix % nx), py = (int)(pix / nx);
     const float fx = (float)px, fy = (float)py;
     float acc[P][CPL];
@@ -459,73 +543,50 @@ __global__ void __launch_bounds__(32 * WARPS) radon_backward_v3(
     for (int h = 0; h < P; ++h)
 #pragma unroll
         for (int c = 0; c < CPL; ++c) acc[h][c] = 0.0f;
-    const ST *col = sino + kblk + lane * CPL;
+    const ST *col = sino + kblk;
     const int64_t angle_stride = (int64_t)ns * sld;
-    for (int a = 0; a < n_angles; ++a, col += angle_stride) {
-        const AngleGeo g = unpack_geo(prm[a]);
-        const float t = __fmaf_rn(g.A, g.rows_are_y ? fx : fy, __fmaf_rn(g.B, g.rows_are_y ? fy : fx, g.T0));
-        const int sf = first_tap<KERNEL>(g, t);
-        const int ntap = taps_of(g, KERNEL, n_taps);
-        if (ntap == 2 && sf >= 0 && sf + 1 < ns) {        // the common case: two taps inside the detector
-            const float w0 = __fmul_rn(g.w, tap_weight<KERNEL>(g, __fsub_rn(t, (float)sf)));
-            const float w1 = __fmul_rn(g.w, tap_weight<KERNEL>(g, __fsub_rn(t, (float)(sf + 1))));
+    if (data[0]) {
+        for (int a = 0; a < n_angles; ++a, col += angle_stride) {
+            const AngleGeo g = unpack_geo(prm[a]);
+            const float t = __fmaf_rn(g.A, g.rows_are_y ? fx : fy, __fmaf_rn(g.B, g.rows_are_y ? fy : fx, g.T0));
+            const int sf = first_tap<KERNEL>(g, t);
+            const int ntap = taps_of(g, KERNEL, n_taps);
+            if (ntap == 2 && sf >= 0 && sf + 1 < ns) {        // the common case: two taps inside the detector
+                const float w0 = __fmul_rn(g.w, tap_weight<KERNEL>(g, __fsub_rn(t, (float)sf)));
+                const float w1 = __fmul_rn(g.w, tap_weight<KERNEL>(g, __fsub_rn(t, (float)(sf + 1))));
 #pragma unroll
-            for (int h = 0; h < P; ++h) {
-                if (!data[h]) continue;
-                float4 a0, a1, b0, b1;
-                ld8(col + h * CPW + (int64_t)sf * sld, a0, a1);
-                ld8(col + h * CPW + (int64_t)(sf + 1) * sld, b0, b1);
-                acc8(acc[h], w0, a0, a1);
-                acc8(acc[h], w1, b0, b1);
+                for (int h = 0; h < P; ++h) {
+                    if (!data[h]) continue;
+                    float4 a0, a1, b0, b1;
+                    ldrow(col + h * CPW + (int64_t)sf * sld, o[h][0], o[h][1], a0, a1);
+                    ldrow(col + h * CPW + (int64_t)(sf + 1) * sld, o[h][0], o[h][1], b0, b1);
+                    acc8(acc[h], w0, a0, a1);
+                    acc8(acc[h], w1, b0, b1);
+                }
+                continue;
             }
-            continue;
-        }
-        for (int i = 0; i < ntap; ++i) {
-            const int s = sf + i;
-            if (s < 0 || s >= ns) continue;
-            const float w = tap_weight<KERNEL>(g, __fsub_rn(t, (float)s));
-            if (w == 0.0f) continue;
-            const float ww = __fmul_rn(g.w, w);
+            for (int i = 0; i < ntap; ++i) {
+                const int s = sf + i;
+                if (s < 0 || s >= ns) continue;
+                const float w = tap_weight<KERNEL>(g, __fsub_rn(t, (float)s));
+                if (w == 0.0f) continue;
+                const float ww = __fmul_rn(g.w, w);
 #pragma unroll
-            for (int h = 0; h < P; ++h) {
-                if (!data[h]) continue;
-                float4 q0, q1;
-                ld8(col + h * CPW + (int64_t)s * sld, q0, q1);
-                acc8(acc[h], ww, q0, q1);
+                for (int h = 0; h < P; ++h) {
+                    if (!data[h]) continue;
+                    float4 q0, q1;
+                    ldrow(col + h * CPW + (int64_t)s * sld, o[h][0], o[h][1], q0, q1);
+                    acc8(acc[h], ww, q0, q1);
+                }
             }
         }
     }
 #pragma unroll
     for (int h = 0; h < P; ++h) {
-        const int k = kblk + h * CPW + lane * CPL;
-        const int64_t o = p * kstride + k;
-        if (MODE == 0) {
-            if (!live[h]) continue;
-            float r[CPL];
+        if (MODE == 1 && !data[h]) continue;
 #pragma unroll
-            for (int c = 0; c < CPL; ++c) r[c] = (data[h] && k + c < kb) ? acc[h][c] : 0.0f;   // padding: 0
-            float4 *d = reinterpret_cast<float4 *>(img + o);
-            d[0] = make_float4(r[0], r[1], r[2], r[3]);
-            d[1] = make_float4(r[4], r[5], r[6], r[7]);
-        } else {
-            if (!data[h]) continue;
-            float xn[CPL];
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-                float4 *xp = reinterpret_cast<float4 *>(img + o) + q;
-                float4 *zp = reinterpret_cast<float4 *>(z + o) + q;
-                float4 xv = *xp, zv = *zp;
-                const float4 tv = __ldg(reinterpret_cast<const float4 *>(T + o) + q);
-                primal_step(xv.x, zv.x, tv.x, (k + 4 * q + 0 < kb) ? acc[h][4 * q + 0] : 0.0f, inv_p, lam);
-                primal_step(xv.y, zv.y, tv.y, (k + 4 * q + 1 < kb) ? acc[h][4 * q + 1] : 0.0f, inv_p, lam);
-                primal_step(xv.z, zv.z, tv.z, (k + 4 * q + 2 < kb) ? acc[h][4 * q + 2] : 0.0f, inv_p, lam);
-                primal_step(xv.w, zv.w, tv.w, (k + 4 * q + 3 < kb) ? acc[h][4 * q + 3] : 0.0f, inv_p, lam);
-                *xp = xv;
-                *zp = zv;
-                xn[4 * q] = xv.x; xn[4 * q + 1] = xv.y; xn[4 * q + 2] = xv.z; xn[4 * q + 3] = xv.w;
-            }
-            if (xb) st8(xb + o, xn);       // the BF16 copy of x the next forward projection reads
-        }
+        for (int r = 0; r < 2; ++r)
+            finish_run<MODE>(img, z, T, xb, p, k[h][r], kstride, kb, acc[h] + 4 * r, inv_p, lam);
     }
 }
 
@@ -852,22 +913,43 @@ extern "C" int dfx_radon_gtable_fill(const float *geo, int n_angles, int nx, int
     return launch_status("radon_gtable_fill");
 }
 
-extern "C" int dfx_radon_forward_gtable(const float *img_k, float *sino_k, const int32_t *row_ptr,
-                                        const int32_t *pixels, const float *weights, const int32_t *angles,
-                                        int n_angles, int n_det, int kstride, int kb, float scale, void *stream)
+template <typename ST>
+static int radon_forward_gtable_any(const float *img_k, ST *sino, int64_t sld, const int32_t *row_ptr,
+                                    const int32_t *pixels, const float *weights, const int32_t *angles, int n_angles,
+                                    int n_det, int kstride, int kb, float scale, void *stream)
 {
-    DFX_REQUIRE(img_k && sino_k && row_ptr && pixels && weights, "radon_forward_gtable: null pointer");
-    DFX_REQUIRE(((uintptr_t)img_k % 16) == 0 && ((uintptr_t)sino_k % 16) == 0 && ((uintptr_t)weights % 16) == 0,
+    DFX_REQUIRE(img_k && sino && row_ptr && pixels && weights, "radon_forward_gtable: null pointer");
+    DFX_REQUIRE(((uintptr_t)img_k % 16) == 0 && ((uintptr_t)sino % 16) == 0 && ((uintptr_t)weights % 16) == 0,
                 "radon_forward_gtable: misaligned arrays");
     DFX_REQUIRE(n_angles >= 0 && n_angles <= 65535 && n_det > 0, "radon_forward_gtable: bad sizes");
     DFX_REQUIRE(kstride > 0 && kstride % CPL == 0 && kb >= 0 && kb <= kstride && cdiv(kstride, CPW) <= 65535,
                 "radon_forward_gtable: kstride (%d) must be a positive multiple of %d and kb (%d) <= kstride",
                 kstride, CPL, kb);
+    DFX_REQUIRE(sld >= kstride && sld % CPL == 0, "radon_forward_gtable: sinogram row stride (%lld) must be a "
+                "multiple of %d >= kstride", (long long)sld, CPL);
     if (n_angles == 0) return DFX_OK;
-    dim3 grid((unsigned)cdiv(cdiv(n_det, GB), WARPS), (unsigned)n_angles, (unsigned)cdiv(kstride, CPW));
-    radon_forward_gtable<<<grid, 32 * WARPS, 0, (cudaStream_t)stream>>>(
-        img_k, sino_k, row_ptr, pixels, reinterpret_cast<const float4 *>(weights), angles, n_det, kstride, kb, scale);
+    dim3 grid((unsigned)cdiv(cdiv(n_det, GB), WARPS / GA), (unsigned)cdiv(n_angles, GA), (unsigned)cdiv(kstride, CPW));
+    radon_forward_gtable<ST><<<grid, 32 * WARPS, 0, (cudaStream_t)stream>>>(
+        img_k, sino, sld, row_ptr, pixels, reinterpret_cast<const float4 *>(weights), angles, n_angles, n_det, kstride,
+        kb, scale);
     return launch_status("radon_forward_gtable");
+}
+
+extern "C" int dfx_radon_forward_gtable(const float *img_k, float *sino_k, const int32_t *row_ptr,
+                                        const int32_t *pixels, const float *weights, const int32_t *angles,
+                                        int n_angles, int n_det, int kstride, int kb, float scale, void *stream)
+{
+    return radon_forward_gtable_any(img_k, sino_k, (int64_t)kstride, row_ptr, pixels, weights, angles, n_angles, n_det,
+                                    kstride, kb, scale, stream);
+}
+
+extern "C" int dfx_radon_forward_gtable_bf16(const float *img_k, void *sino_bf16, int64_t sino_ld,
+                                             const int32_t *row_ptr, const int32_t *pixels, const float *weights,
+                                             const int32_t *angles, int n_angles, int n_det, int kstride, int kb,
+                                             float scale, void *stream)
+{
+    return radon_forward_gtable_any(img_k, reinterpret_cast<__nv_bfloat16 *>(sino_bf16), sino_ld, row_ptr, pixels,
+                                    weights, angles, n_angles, n_det, kstride, kb, scale, stream);
 }
 
 extern "C" int dfx_radon_dtable_fill(const float *geo, int n_angles, int nx, int ny, int n_det, int kernel,

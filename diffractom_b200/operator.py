@@ -36,7 +36,7 @@ AUTO_FFT_PIXELS = 400 * 400   # projector="auto": the Fourier-slice projector fo
 SPARSE_MIN_BATCHES = 4    # sparse modes: at least this many batches (SPFO:135)
 CAND_BYTES = 2 + 4 + 4 + 4 + 4          # per candidate / non-zero scratch of the reference's generator
 NNZ_BYTES = 2 + 4 + 4 + 2 + 4 + 2 + 4   # (pf_generate.py:29-30), used by the batch-size rule
-GTABLE_MIN_ANGLES = 64                   # float32 forwards of this many angles read the grouped table
+GTABLE_MIN_WARPS = 4 * 148 * 32          # forwards of a scan with this many grouped-table warps read the grouped table
 KSTRIDE_ALIGN = 16                       # channel stride of the batch buffers (16 channels per tensor-memory load)
 
 
@@ -381,12 +381,17 @@ class SinglePhaseForwardOperator:
         om_ptr = None if om is None else om.data_ptr()
         rp, ent = (self._ray_rp, self._ray_ent) if ray is None else ray[:2]
         grp = self._ray_grp if ray is None else (ray[3] if len(ray) > 3 else None)
-        # the grouped table has a quarter of the warps: for a few angles (a subset) the per-bin one fills the GPU
-        # better (at 256 x 256, 1024 channels and 18 angles: 0.56 ms per-bin, 0.63 to 0.67 ms grouped)
-        if sld is None and grp is not None and n_ang >= GTABLE_MIN_ANGLES:
-            self._call("dfx_radon_forward_gtable", src_ptr, dst_ptr, grp[0].data_ptr(), grp[1].data_ptr(),
-                       grp[2].data_ptr(), om_ptr, n_ang, self.My, self.Kstride, kb, float(self.radon_geo.scale),
-                       self._s())
+        # a scan's consecutive angles share their pixels in L1 through the grouped table, a subset's do not (18 angles
+        # at 256 x 256 pixels, 1012 channels: 0.75 ms grouped, 0.44 ms per-bin; all 360: 6.6 and 7.2 ms). It has a
+        # quarter of the warps: below about four waves of them the per-bin table is as fast (180 angles of 99 x 99
+        # pixels, 4 waves: 0.556 and 0.560 ms) or faster (91 angles of 131 x 131 pixels, 333 channels, 1.3 waves: 0.31
+        # and 0.26 ms; 90 of 48 x 48, half a wave: 0.069 and 0.048 ms)
+        warps = n_ang * -(-self.My // 4) * -(-self.Kstride // 256)
+        if grp is not None and m is None and warps >= GTABLE_MIN_WARPS:
+            out = (dst_ptr,) if sld is None else (dst_ptr, sld)
+            self._call("dfx_radon_forward_gtable" if sld is None else "dfx_radon_forward_gtable_bf16", src_ptr, *out,
+                       grp[0].data_ptr(), grp[1].data_ptr(), grp[2].data_ptr(), om_ptr, n_ang, self.My, self.Kstride,
+                       kb, float(self.radon_geo.scale), self._s())
         elif sld is None:
             self._call("dfx_radon_forward_table", src_ptr, dst_ptr, rp.data_ptr(), ent.data_ptr(),
                        om_ptr, n_ang, self.My, self.Kstride, kb, float(self.radon_geo.scale), self._s())

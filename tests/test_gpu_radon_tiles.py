@@ -1,0 +1,98 @@
+"""The native projector's kernels at the sizes where their work split can go wrong (GPU): channel counts around the 256
+of a warp and its two runs of 128, bins around the groups of four, angle counts around a block's, image widths around a
+tile's, detectors narrower than the image (taps at its edge), both footprints."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+# (nx, ny, bins, angles, kb, kstride)
+SIZES = [(5, 4, 6, 3, 1, 8), (8, 7, 9, 9, 12, 16), (17, 21, 11, 13, 127, 128), (19, 16, 24, 8, 130, 136),
+         (33, 30, 41, 17, 250, 256), (16, 18, 15, 16, 257, 264), (23, 9, 26, 7, 500, 504), (12, 35, 37, 5, 1000, 1008)]
+
+
+def _geometry(nx, ny, bins, angles, kernel):
+    from diffractom_b200.geometry import radon_geometry
+    ang = (np.arange(angles) + 0.5) * np.pi / angles
+    return radon_geometry(ang, nx, ny, bins, float(max(nx, ny)), float(bins), 0.3, np.pi / angles, kernel)
+
+
+def _tables(rg, nx, ny, bins, kid, group):
+    from diffractom_b200 import _lib
+    s = torch.cuda.current_stream().cuda_stream
+    geo = torch.as_tensor(rg.geo, device="cuda")
+    R = len(rg.geo)
+    kind = "gtable" if group else "table"
+    cnt = torch.empty(R * (-(-bins // 4) if group else bins), dtype=torch.int32, device="cuda")
+    _lib.call(f"dfx_radon_{kind}_count", geo.data_ptr(), R, nx, ny, bins, kid, None, cnt.data_ptr(), s)
+    rp = torch.zeros(cnt.numel() + 1, dtype=torch.int32, device="cuda")
+    rp[1:] = cnt.cumsum(0)
+    n = max(int(rp[-1].item()), 1)
+    if not group:
+        ent = torch.empty(2 * n, dtype=torch.int32, device="cuda")
+        _lib.call("dfx_radon_table_fill", geo.data_ptr(), R, nx, ny, bins, kid, None, rp.data_ptr(), ent.data_ptr(), s)
+        return rp, ent
+    pix, w = torch.empty(n, dtype=torch.int32, device="cuda"), torch.empty((n, 4), device="cuda")
+    _lib.call("dfx_radon_gtable_fill", geo.data_ptr(), R, nx, ny, bins, kid, None, rp.data_ptr(), pix.data_ptr(),
+              w.data_ptr(), s)
+    return rp, pix, w
+
+
+@pytest.mark.parametrize("kernel", ["trapezoid", "hat"])
+@pytest.mark.parametrize("size", SIZES, ids=str)
+def test_forward_tables_equal_the_footprint_forward(size, kernel):
+    """Per-bin and grouped table forwards, float32 and BF16 rows, all angles and a list: dfx_radon_forward's bits
+    (the BF16 rows its values rounded once); padding channels are not read."""
+    from diffractom_b200 import _lib
+    nx, ny, bins, R, kb, ks = size
+    rg = _geometry(nx, ny, bins, R, kernel)
+    kid, scale, s = int(kernel == "trapezoid"), float(rg.scale), torch.cuda.current_stream().cuda_stream
+    geo = torch.as_tensor(rg.geo, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(3)
+    img = torch.randn((nx * ny, ks), generator=g, device="cuda")
+    img[:, kb:] = float("nan")
+    ref = torch.empty((R, bins, ks), device="cuda")
+    _lib.call("dfx_radon_forward", img.data_ptr(), ref.data_ptr(), geo.data_ptr(), R, nx, ny, bins, ks, kb, kid, scale, s)
+    assert torch.isfinite(ref).all() and not ref[:, :, kb:].any()
+    rp, ent = _tables(rg, nx, ny, bins, kid, False)
+    grp = _tables(rg, nx, ny, bins, kid, True)
+    some = torch.arange(R - 1, -1, -2, dtype=torch.int32, device="cuda")
+    ld = ks + 8
+    for om in (None, some):
+        n = R if om is None else om.numel()
+        want = ref if om is None else ref[om.long()]
+        op = None if om is None else om.data_ptr()
+        out, outb = torch.empty((n, bins, ks), device="cuda"), torch.empty((n, bins, ld), dtype=torch.bfloat16, device="cuda")
+        _lib.call("dfx_radon_forward_table", img.data_ptr(), out.data_ptr(), rp.data_ptr(), ent.data_ptr(), op, n, bins,
+                  ks, kb, scale, s)
+        assert torch.equal(out, want)
+        _lib.call("dfx_radon_forward_table_bf16", img.data_ptr(), outb.data_ptr(), ld, rp.data_ptr(), ent.data_ptr(), op,
+                  n, bins, ks, kb, scale, s)
+        assert torch.equal(outb[:, :, :ks], want.to(torch.bfloat16))
+        out.zero_(), outb.zero_()
+        _lib.call("dfx_radon_forward_gtable", img.data_ptr(), out.data_ptr(), *(t.data_ptr() for t in grp), op, n, bins,
+                  ks, kb, scale, s)
+        assert torch.equal(out, want)
+        _lib.call("dfx_radon_forward_gtable_bf16", img.data_ptr(), outb.data_ptr(), ld, *(t.data_ptr() for t in grp), op,
+                  n, bins, ks, kb, scale, s)
+        assert torch.equal(outb[:, :, :ks], want.to(torch.bfloat16))
+
+
+def test_bf16_image_table_forward_equals_the_float32_one():
+    """A BF16 image (widened exactly) through the per-bin table: the float32 forward of the same values."""
+    from diffractom_b200 import _lib
+    for nx, ny, bins, R, kb, ks in SIZES:
+        rg = _geometry(nx, ny, bins, R, "trapezoid")
+        s = torch.cuda.current_stream().cuda_stream
+        g = torch.Generator(device="cuda").manual_seed(4)
+        img = torch.randn((nx * ny, ks), generator=g, device="cuda").to(torch.bfloat16)
+        img32 = img.float()
+        rp, ent = _tables(rg, nx, ny, bins, 1, False)
+        a = torch.empty((R, bins, ks), dtype=torch.bfloat16, device="cuda")
+        b = torch.empty_like(a)
+        _lib.call("dfx_radon_forward_table_bf16_bf16", img.data_ptr(), a.data_ptr(), ks, rp.data_ptr(), ent.data_ptr(),
+                  None, R, bins, ks, kb, float(rg.scale), s)
+        _lib.call("dfx_radon_forward_table_bf16", img32.data_ptr(), b.data_ptr(), ks, rp.data_ptr(), ent.data_ptr(), None,
+                  R, bins, ks, kb, float(rg.scale), s)
+        assert torch.equal(a, b)
