@@ -96,3 +96,69 @@ def test_bf16_image_table_forward_equals_the_float32_one():
         _lib.call("dfx_radon_forward_table_bf16", img32.data_ptr(), b.data_ptr(), ks, rp.data_ptr(), ent.data_ptr(), None,
                   R, bins, ks, kb, float(rg.scale), s)
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("kernel", ["trapezoid", "hat"])
+@pytest.mark.parametrize("size", SIZES, ids=str)
+def test_backprojection_of_whole_images_equals_the_pixel_lists(size, kernel):
+    """dfx_radon_backward (rows of pixels sharing bins) = dfx_radon_backward_pixels over every pixel (pixel by pixel),
+    bit for bit: float32 and BF16 rows with their own stride, padding channels 0; dfx_radon_backward_spdhg = the
+    backprojection followed by dfx_spdhg_primal_update, the padding channels of x, z kept."""
+    from diffractom_b200 import _lib
+    nx, ny, bins, R, kb, ks = size
+    rg = _geometry(nx, ny, bins, R, kernel)
+    kid, nt, s = int(kernel == "trapezoid"), int(rg.n_taps), torch.cuda.current_stream().cuda_stream
+    assert nt == 2
+    geo = torch.as_tensor(rg.geo, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(5)
+    sino = torch.randn((R, bins, ks), generator=g, device="cuda")
+    pix = torch.arange(nx * ny, dtype=torch.int32, device="cuda")
+    want, out = torch.empty((nx * ny, ks), device="cuda"), torch.empty((nx * ny, ks), device="cuda")
+
+    def pixels(src):
+        _lib.call("dfx_radon_backward_pixels", src.data_ptr(), want.data_ptr(), geo.data_ptr(), R, nx, ny, bins, ks, kb,
+                  kid, nt, pix.data_ptr(), nx * ny, s)
+
+    pixels(sino)
+    _lib.call("dfx_radon_backward", sino.data_ptr(), out.data_ptr(), geo.data_ptr(), R, nx, ny, bins, ks, kb, kid, nt, s)
+    assert torch.equal(out, want) and want.any() and not want[:, kb:].any()
+    # the primal step in the epilogue
+    x, z, T = (torch.rand((nx * ny, ks), generator=g, device="cuda") for _ in range(3))
+    x[:, kb:] = z[:, kb:] = T[:, kb:] = 0
+    xr, zr = x.clone(), z.clone()
+    _lib.call("dfx_spdhg_primal_update", xr.data_ptr(), zr.data_ptr(), T.data_ptr(), want.data_ptr(), 7.0, 0.25,
+              x.numel(), s)
+    _lib.call("dfx_radon_backward_spdhg", sino.data_ptr(), geo.data_ptr(), R, nx, ny, bins, ks, kb, kid, nt, x.data_ptr(),
+              z.data_ptr(), T.data_ptr(), 7.0, 0.25, s)
+    assert torch.equal(x, xr) and torch.equal(z, zr)
+    # BF16 rows of a wider sinogram
+    ld = ks + 8
+    sb = torch.randn((R, bins, ld), generator=g, device="cuda").to(torch.bfloat16)
+    pixels(sb[:, :, :ks].float().contiguous())
+    _lib.call("dfx_radon_backward_bf16", sb.data_ptr(), ld, out.data_ptr(), geo.data_ptr(), R, nx, ny, bins, ks, kb, kid,
+              nt, s)
+    assert torch.equal(out, want)
+
+
+def test_backprojection_with_more_than_two_taps():
+    """Pixels wider than the bins (three or four taps a pixel): the general kernel, against the forward's transpose
+    in float64 (2 x 20 angles x 4 taps of float32 rounding)."""
+    from diffractom_b200 import _lib
+    from diffractom_b200.geometry import radon_geometry
+    nx, ny, bins, R, kb, ks = 9, 11, 31, 20, 40, 48
+    ang = (np.arange(R) + 0.5) * np.pi / R
+    rg = radon_geometry(ang, nx, ny, bins, 28.0, float(bins), 0.0, 1.0, "trapezoid")
+    assert rg.n_taps > 2
+    s = torch.cuda.current_stream().cuda_stream
+    geo = torch.as_tensor(rg.geo, device="cuda")
+    eye = torch.zeros((nx * ny, 104), device="cuda")
+    eye[torch.arange(nx * ny), torch.arange(nx * ny)] = 1.0
+    A = torch.empty((R, bins, 104), device="cuda")
+    _lib.call("dfx_radon_forward", eye.data_ptr(), A.data_ptr(), geo.data_ptr(), R, nx, ny, bins, 104, 104, 1, 1.0, s)
+    sino = torch.randn((R, bins, ks), device="cuda")
+    out = torch.empty((nx * ny, ks), device="cuda")
+    _lib.call("dfx_radon_backward", sino.data_ptr(), out.data_ptr(), geo.data_ptr(), R, nx, ny, bins, ks, kb, 1,
+              int(rg.n_taps), s)
+    want = torch.einsum("abp,abk->pk", A[:, :, :nx * ny].double(), sino.double())
+    bound = torch.einsum("abp,abk->pk", A[:, :, :nx * ny].double().abs(), sino.double().abs()) * 2 * R * 4 * 2.0 ** -24
+    assert ((out.double() - want).abs()[:, :kb] <= bound[:, :kb]).all() and not out[:, kb:].any()
