@@ -19,6 +19,7 @@
 #include <cuda_bf16.h>
 
 #include "dfx_common.cuh"
+#include "transpose.cuh"
 
 namespace dfx {
 
@@ -790,47 +791,6 @@ __global__ void batch_support_kernel(float *__restrict__ x, const float *__restr
     }
 }
 
-// (Ktot, npix) <-> (npix, kstride) channel transposes through a 32 x 33 shared tile.
-constexpr int TT = 32;
-
-__global__ void __launch_bounds__(TT * 8) gather_kernel(const float *__restrict__ coeffs, float *__restrict__ img,
-                                                        int64_t npix, int k0, int kb, int kstride)
-{
-    __shared__ float tile[TT][TT + 1];
-    const int64_t p0 = (int64_t)blockIdx.x * TT;
-    const int q0 = blockIdx.y * TT;
-    for (int j = threadIdx.y; j < TT; j += 8) {            // read: pixels contiguous
-        const int64_t p = p0 + threadIdx.x;
-        const int q = q0 + j;
-        tile[j][threadIdx.x] = (p < npix && q < kb) ? coeffs[(int64_t)(k0 + q) * npix + p] : 0.0f;
-    }
-    __syncthreads();
-    for (int j = threadIdx.y; j < TT; j += 8) {            // write: channels contiguous
-        const int64_t p = p0 + j;
-        const int q = q0 + threadIdx.x;
-        if (p < npix && q < kstride) img[p * kstride + q] = tile[threadIdx.x][j];
-    }
-}
-
-__global__ void __launch_bounds__(TT * 8) scatter_kernel(const float *__restrict__ img, float *__restrict__ coeffs,
-                                                         int64_t npix, int k0, int kb, int kstride)
-{
-    __shared__ float tile[TT][TT + 1];
-    const int64_t p0 = (int64_t)blockIdx.x * TT;
-    const int q0 = blockIdx.y * TT;
-    for (int j = threadIdx.y; j < TT; j += 8) {            // read: channels contiguous
-        const int64_t p = p0 + j;
-        const int q = q0 + threadIdx.x;
-        tile[j][threadIdx.x] = (p < npix && q < kstride) ? img[p * kstride + q] : 0.0f;
-    }
-    __syncthreads();
-    for (int j = threadIdx.y; j < TT; j += 8) {            // write: pixels contiguous
-        const int64_t p = p0 + threadIdx.x;
-        const int q = q0 + j;
-        if (p < npix && q < kb) coeffs[(int64_t)(k0 + q) * npix + p] = tile[threadIdx.x][j];
-    }
-}
-
 static int check_radon_args(const void *in, const void *out, const void *geo, int n_angles, int nx, int ny,
                             int n_det, int kstride, int kb, int kernel)
 {
@@ -1195,10 +1155,8 @@ extern "C" int dfx_gather_channels(const float *coeffs, float *img_k, int64_t np
 {
     DFX_REQUIRE(coeffs && img_k, "gather: null pointer");
     DFX_REQUIRE(npix > 0 && k0 >= 0 && kb >= 0 && kb <= kstride, "gather: bad sizes");
-    dim3 grid((unsigned)cdiv(npix, TT), (unsigned)cdiv(kstride, TT));
-    DFX_REQUIRE(grid.y <= 65535u, "gather: kstride too large");
-    gather_kernel<<<grid, dim3(TT, 8), 0, (cudaStream_t)stream>>>(coeffs, img_k, npix, k0, kb, kstride);
-    return launch_status("gather_channels");
+    return launch_transpose(coeffs + (int64_t)k0 * npix, npix, 0, nullptr, 0, img_k, kstride, 0, kb, kstride, npix, 1,
+                            (cudaStream_t)stream);
 }
 
 extern "C" int dfx_scatter_channels(const float *img_k, float *coeffs, int64_t npix, int k0, int kb, int kstride,
@@ -1207,8 +1165,6 @@ extern "C" int dfx_scatter_channels(const float *img_k, float *coeffs, int64_t n
     DFX_REQUIRE(coeffs && img_k, "scatter: null pointer");
     DFX_REQUIRE(npix > 0 && k0 >= 0 && kb >= 0 && kb <= kstride, "scatter: bad sizes");
     if (kb == 0) return DFX_OK;
-    dim3 grid((unsigned)cdiv(npix, TT), (unsigned)cdiv(kb, TT));
-    DFX_REQUIRE(grid.y <= 65535u, "scatter: kb too large");
-    scatter_kernel<<<grid, dim3(TT, 8), 0, (cudaStream_t)stream>>>(img_k, coeffs, npix, k0, kb, kstride);
-    return launch_status("scatter_channels");
+    return launch_transpose(img_k, kstride, 0, nullptr, 0, coeffs + (int64_t)k0 * npix, npix, 0, npix, npix, kb, 1,
+                            (cudaStream_t)stream);
 }

@@ -14,6 +14,7 @@
 // whole 128-byte segment of the column per 32 lines (spmm_forward_zt_kernel, spmm_adjoint_zt_kernel); their sums
 // are the kernels' above bit for bit.
 #include "dfx_common.cuh"
+#include "transpose.cuh"
 
 #include <algorithm>
 
@@ -415,10 +416,11 @@ __global__ void __launch_bounds__(SP_ROWS) spmm_forward_b4_kernel(
 // ---- blocked forward over the lines-fastest sinogram ----
 // zt[s][k][y] (line stride ly = 32 * groups, lines my .. ly - 1 zero) is the Radon output of one launch's angles with
 // the detector lines fastest. A warp applies one block row (four eta bins of one ring) of one angle at a time to up
-// to 32 ZT_G lines: lane l holds the lines y0 + l + 32 t. Per entry the warp reads the entry once (the same address in
-// every lane) and one coalesced 128-byte segment of Z column k per 32 lines, four entries in flight, and applies the
-// entry's four values with paired fused multiply-adds (fma.rn.f32x2: two IEEE fmaf in one instruction, lines t and
-// t + 1). A block of 8 warps owns the block rows of nb consecutive eta blocks, all rings (nb * P <= 16 rows; one eta
+// to 32 ZT_G lines (ZtLines). Per entry the warp reads the entry once (the same address in every lane) and the lines
+// of Z column k in 512-byte segments, several entries in flight, and applies the entry's four values with paired fused
+// multiply-adds (fma.rn.f32x2: two IEEE fmaf in one instruction, lines t and t + 1). Instructions bounded it: with a
+// 4-byte load per 32 lines, each guarded, 92 per entry, now 65 (2.27 -> 1.86 ms for the 360 angles of 256 x 256 pixels,
+// 1012 channels, transposes in; 0.64 -> 0.56 for the 180 of 99 x 99); what is left is L2 latency at 24 warps. A block of 8 warps owns the block rows of nb consecutive eta blocks, all rings (nb * P <= 16 rows; one eta
 // block above 16 rings), whose outputs j = 4 cb P .. 4 (cb + nb) P - 1 are contiguous in a data row. The rows differ
 // in length, so the warps take them longest first from a shared counter instead of one row each: the block no longer
 // waits for its longest row with most warps idle. The sums go to shared memory; the block's data row segments, put in
@@ -426,26 +428,9 @@ __global__ void __launch_bounds__(SP_ROWS) spmm_forward_b4_kernel(
 // per output run over the block row's entries in order with fmaf, each added once to the data row, as in
 // spmm_forward_b4_kernel: the results are that kernel's (and the CSR kernel's) bit for bit.
 constexpr int ZT_G = 9;                  // 32-line groups per warp at most (288 lines)
-constexpr int ZT_U = 4;                  // entries in flight per warp
-constexpr int ZT_TR = 32;                // transpose tile
-
-// zt[s][k][y] = sino[s][y][k] (k < kb, y < my; zero for my <= y < ly)
-__global__ void __launch_bounds__(256) zt_transpose_kernel(const float *__restrict__ sino, float *__restrict__ zt,
-                                                           int my, int ly, int kstride, int kb)
-{
-    __shared__ float tile[ZT_TR][ZT_TR + 1];
-    const int s = blockIdx.z, k0 = blockIdx.x * ZT_TR, y0 = blockIdx.y * ZT_TR;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    for (int yy = ty; yy < ZT_TR; yy += 8) {
-        const int y = y0 + yy, k = k0 + tx;
-        tile[yy][tx] = (y < my && k < kb) ? __ldg(sino + ((int64_t)s * my + y) * kstride + k) : 0.0f;
-    }
-    __syncthreads();
-    for (int kk = ty; kk < ZT_TR; kk += 8) {
-        const int k = k0 + kk;
-        if (k < kb) zt[((int64_t)s * kb + k) * ly + y0 + tx] = tile[tx][kk];
-    }
-}
+// entries in flight per warp for MT line groups
+constexpr int zt_uf(int mt, bool wide) { return mt <= 2 ? 8 : wide ? 3 : 4; }
+constexpr int zt_ua(int mt) { return mt <= 2 ? 8 : 4; }
 
 // a0 = fmaf(v, z0, a0), a1 = fmaf(v, z1, a1) in one instruction (same rounding as two fmaf)
 __device__ __forceinline__ void fma_pair(float &a0, float &a1, float v, float z0, float z1)
@@ -455,15 +440,61 @@ __device__ __forceinline__ void fma_pair(float &a0, float &a1, float v, float z0
     a1 = r.y;
 }
 
+// The 32 MT lines of a warp: lane l holds, for every whole group of 128 lines, the four lines 128 g + 4 l .. + 3 (one
+// 16-byte load of the warp reads 512 contiguous bytes), and of the MT % 4 groups left two neighbouring lines (8-byte
+// loads) and one (4-byte). Value t of lane l stands in shared memory at slot 32 t + l.
+template <int MT>
+struct ZtLines {
+    static constexpr int Q = MT / 4, R = MT % 4;
+    const float *p4, *p2, *p1;
+    __device__ __forceinline__ ZtLines(const float *z, int lane)
+        : p4(z + 4 * lane), p2(z + 128 * Q + 2 * lane), p1(z + 128 * Q + (R >= 2 ? 64 : 0) + lane) {}
+    // z = the lane's lines of the column at byte offset b
+    __device__ __forceinline__ void load(uint32_t b, float (&z)[MT]) const
+    {
+#pragma unroll
+        for (int g = 0; g < Q; ++g) {
+            const float4 v = __ldg(reinterpret_cast<const float4 *>(reinterpret_cast<const char *>(p4) + b) + 32 * g);
+            z[4 * g] = v.x;
+            z[4 * g + 1] = v.y;
+            z[4 * g + 2] = v.z;
+            z[4 * g + 3] = v.w;
+        }
+        if constexpr (R >= 2) {
+            const float2 v = __ldg(reinterpret_cast<const float2 *>(reinterpret_cast<const char *>(p2) + b));
+            z[4 * Q] = v.x;
+            z[4 * Q + 1] = v.y;
+        }
+        if constexpr (R & 1) z[MT - 1] = __ldg(reinterpret_cast<const float *>(reinterpret_cast<const char *>(p1) + b));
+    }
+    static __device__ __forceinline__ int slot(int y)
+    {
+        if (y < 128 * Q) return 32 * (4 * (y >> 7) + (y & 3)) + ((y & 127) >> 2);
+        const int r = y - 128 * Q;
+        if (R >= 2 && r < 64) return 32 * (4 * Q + (r & 1)) + (r >> 1);
+        return 32 * (MT - 1) + r - (R >= 2 ? 64 : 0);
+    }
+};
+
+// acc += v z on the lane's lines
+template <int MT>
+__device__ __forceinline__ void fma_lines(float (&acc)[MT], float v, const float (&z)[MT])
+{
+#pragma unroll
+    for (int t = 0; t + 1 < MT; t += 2) fma_pair(acc[t], acc[t + 1], v, z[t], z[t + 1]);
+    if (MT & 1) acc[MT - 1] = __fmaf_rn(v, z[MT - 1], acc[MT - 1]);
+}
+
 constexpr int ZT_ROWS_MAX = 32;         // block rows per block at most (one eta block of 32 rings)
 constexpr int ZT_NB_LINES = 9;           // data row lines read per batch in the write-back
 
-template <int MT>
-__global__ void __launch_bounds__(256, 2) spmm_forward_zt_kernel(
+template <int MT, bool WIDE>
+__global__ void __launch_bounds__(256, WIDE ? 3 : 2) spmm_forward_zt_kernel(
     const float *__restrict__ zt, const int32_t *__restrict__ fb_ptr, const uint16_t *__restrict__ fb_k,
     const float4 *__restrict__ fb_v, const uint8_t *__restrict__ fb_mask, float *__restrict__ data,
     const int32_t *__restrict__ omegas, int r0, int my, int ly, int P, int C, int ncb, int nb, int kb)
 {
+    constexpr int U = zt_uf(MT, WIDE);
     extern __shared__ __align__(16) float s_out[];    // [32 MT][width + 1]: the block's sums
     __shared__ uint8_t s_own[FB_W * ZT_ROWS_MAX];      // output j of the block written (its bin's row has entries)
     __shared__ int s_order[ZT_ROWS_MAX];               // the block's rows, longest first
@@ -472,8 +503,10 @@ __global__ void __launch_bounds__(256, 2) spmm_forward_zt_kernel(
     const int s = blockIdx.z;
     const int r = omegas ? __ldg(omegas + s) : r0 + s;
     const int ngroups = ly >> 5;
-    const int g0 = blockIdx.y * MT;                   // first 32-line group of the block
-    const int y0 = g0 * 32;
+    // first 32-line group of the block; the last block of a column of several starts MT groups before the end and
+    // leaves the lines it shares with the one before to that one
+    const int g0 = min((int)blockIdx.y * MT, ngroups - MT);
+    const int y0 = g0 * 32, yskip = ((int)blockIdx.y * MT - g0) * 32;
     const int cb0 = blockIdx.x * nb;
     const int nrows = nb * P;                         // row q: eta block cb0 + q / P, ring q % P
     const int width = FB_W * nb * P, wp = width + 1;
@@ -484,7 +517,7 @@ __global__ void __launch_bounds__(256, 2) spmm_forward_zt_kernel(
     float *drow = data + ((int64_t)r * my + y0) * cp + j0;
     // the data row segments into L2 while the rows are summed (read and written back at the end)
     const int lines = (wj + 31) >> 5;
-    for (int idx = tid; idx < ny * lines; idx += blockDim.x) {
+    for (int idx = yskip * lines + tid; idx < ny * lines; idx += blockDim.x) {
         const int yl = idx / lines, c = idx - yl * lines;
         asm volatile("prefetch.global.L2 [%0];" ::"l"(drow + (int64_t)yl * cp + 32 * c));
     }
@@ -507,65 +540,75 @@ __global__ void __launch_bounds__(256, 2) spmm_forward_zt_kernel(
         if (lane == 0) s_next = 0;
     }
     __syncthreads();
-    const float *zs = zt + (int64_t)s * kb * ly + y0 + lane;
-    while (true) {
+    const ZtLines<MT> zl(zt + (int64_t)s * kb * ly + y0, lane);
+    const uint32_t col_b = (uint32_t)ly * 4u;
+    // the next row's place in the block and its entries' range, fetched while the current one is summed
+    int jn = 0, in = 0, en = 0, mn = 0;
+    auto fetch = [&]() {
         int idx = 0;
         if (lane == 0) idx = atomicAdd(&s_next, 1);
         idx = __shfl_sync(0xffffffffu, idx, 0);
-        if (idx >= nrows) break;
+        jn = -1;
+        if (idx >= nrows) return;
         const int q = s_order[idx], cbw = q / P, p = q - cbw * P, cb = cb0 + cbw;
-        if (cb >= ncb) continue;
+        jn = FB_W * cbw * P + p;                      // local j of bin u: (4 cbw + u) P + p
+        in = en = mn = 0;
+        if (cb >= ncb) return;
         const int64_t g = (int64_t)r * P * ncb + (int64_t)cb * P + p;
-        int i = __ldg(fb_ptr + g);
-        const int e = __ldg(fb_ptr + g + 1);
-        const int m = __ldg(fb_mask + g);
+        in = __ldg(fb_ptr + g);
+        en = __ldg(fb_ptr + g + 1);
+        mn = __ldg(fb_mask + g);
+    };
+    fetch();
+    while (jn >= 0) {
+        const int jl = jn, e = en, m = mn;
+        int i = in;
         float acc[FB_W][MT];
 #pragma unroll
         for (int u = 0; u < FB_W; ++u)
 #pragma unroll
             for (int t = 0; t < MT; ++t) acc[u][t] = 0.0f;
-        int kq[ZT_U];
-        float4 vq[ZT_U];
+        uint32_t kq[U];
+        float4 vq[U];
+        if (i + U <= e) {
 #pragma unroll
-        for (int qq = 0; qq < ZT_U; ++qq) {
-            kq[qq] = i + qq < e ? __ldg(fb_k + i + qq) : 0;
-            vq[qq] = i + qq < e ? __ldg(fb_v + i + qq) : make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int qq = 0; qq < U; ++qq) {
+                kq[qq] = __ldg(fb_k + i + qq);
+                vq[qq] = __ldg(fb_v + i + qq);
+            }
         }
-        for (; i < e; i += ZT_U) {
-            float4 vc[ZT_U];
-            float z[ZT_U][MT];
+        fetch();
+        for (; i + U <= e; i += U) {
+            float4 vc[U];
+            float z[U][MT];
 #pragma unroll
-            for (int qq = 0; qq < ZT_U; ++qq) {
+            for (int qq = 0; qq < U; ++qq) {
                 vc[qq] = vq[qq];
-                const float *zc = zs + (int64_t)kq[qq] * ly;
-#pragma unroll
-                for (int t = 0; t < MT; ++t) z[qq][t] = g0 + t < ngroups ? __ldg(zc + 32 * t) : 0.0f;
+                zl.load(kq[qq] * col_b, z[qq]);
             }
 #pragma unroll
-            for (int qq = 0; qq < ZT_U; ++qq) {        // the next entries' loads go out while these are applied
-                kq[qq] = i + ZT_U + qq < e ? __ldg(fb_k + i + ZT_U + qq) : 0;
-                vq[qq] = i + ZT_U + qq < e ? __ldg(fb_v + i + ZT_U + qq) : make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int qq = 0; qq < U; ++qq) {       // the next entries' loads go out while these are applied
+                const int f = min(i + U + qq, e - 1);
+                kq[qq] = __ldg(fb_k + f);
+                vq[qq] = __ldg(fb_v + f);
             }
 #pragma unroll
-            for (int qq = 0; qq < ZT_U; ++qq) {
-                if (i + qq < e) {
-#pragma unroll
-                    for (int t = 0; t + 1 < MT; t += 2) {
-                        fma_pair(acc[0][t], acc[0][t + 1], vc[qq].x, z[qq][t], z[qq][t + 1]);
-                        fma_pair(acc[1][t], acc[1][t + 1], vc[qq].y, z[qq][t], z[qq][t + 1]);
-                        fma_pair(acc[2][t], acc[2][t + 1], vc[qq].z, z[qq][t], z[qq][t + 1]);
-                        fma_pair(acc[3][t], acc[3][t + 1], vc[qq].w, z[qq][t], z[qq][t + 1]);
-                    }
-                    if (MT & 1) {
-                        acc[0][MT - 1] = __fmaf_rn(vc[qq].x, z[qq][MT - 1], acc[0][MT - 1]);
-                        acc[1][MT - 1] = __fmaf_rn(vc[qq].y, z[qq][MT - 1], acc[1][MT - 1]);
-                        acc[2][MT - 1] = __fmaf_rn(vc[qq].z, z[qq][MT - 1], acc[2][MT - 1]);
-                        acc[3][MT - 1] = __fmaf_rn(vc[qq].w, z[qq][MT - 1], acc[3][MT - 1]);
-                    }
-                }
+            for (int qq = 0; qq < U; ++qq) {
+                fma_lines<MT>(acc[0], vc[qq].x, z[qq]);
+                fma_lines<MT>(acc[1], vc[qq].y, z[qq]);
+                fma_lines<MT>(acc[2], vc[qq].z, z[qq]);
+                fma_lines<MT>(acc[3], vc[qq].w, z[qq]);
             }
         }
-        const int jl = FB_W * cbw * P + p;            // local j of bin u: (4 cbw + u) P + p
+        for (; i < e; ++i) {
+            const float4 v = __ldg(fb_v + i);
+            float z[MT];
+            zl.load(__ldg(fb_k + i) * col_b, z);
+            fma_lines<MT>(acc[0], v.x, z);
+            fma_lines<MT>(acc[1], v.y, z);
+            fma_lines<MT>(acc[2], v.z, z);
+            fma_lines<MT>(acc[3], v.w, z);
+        }
 #pragma unroll
         for (int u = 0; u < FB_W; ++u) {
 #pragma unroll
@@ -578,7 +621,7 @@ __global__ void __launch_bounds__(256, 2) spmm_forward_zt_kernel(
     const int rows_per_pass = blockDim.x / width;     // at least 2: width <= 128
     const int tj = tid % width, ty = tid / width;
     if (ty < rows_per_pass && s_own[tj]) {
-        for (int yb = ty; yb < ny; yb += ZT_NB_LINES * rows_per_pass) {
+        for (int yb = yskip + ty; yb < ny; yb += ZT_NB_LINES * rows_per_pass) {
             float old[ZT_NB_LINES];
 #pragma unroll
             for (int n = 0; n < ZT_NB_LINES; ++n) {
@@ -588,7 +631,7 @@ __global__ void __launch_bounds__(256, 2) spmm_forward_zt_kernel(
 #pragma unroll
             for (int n = 0; n < ZT_NB_LINES; ++n) {
                 const int yl = yb + n * rows_per_pass;
-                if (yl < ny) drow[(int64_t)yl * cp + tj] = old[n] + s_out[yl * wp + tj];
+                if (yl < ny) drow[(int64_t)yl * cp + tj] = old[n] + s_out[ZtLines<MT>::slot(yl) * wp + tj];
             }
         }
     }
@@ -597,91 +640,74 @@ __global__ void __launch_bounds__(256, 2) spmm_forward_zt_kernel(
 // ---- adjoint over the lines-fastest data rows ----
 // dt[s][j][y] (line stride ly, lines my .. ly - 1 zero): the data rows of one launch's angles with the detector lines
 // fastest. A warp owns kw (1, 2 or 4) consecutive orientation rows k of one angle, one after the other, and up to
-// 32 ZT_G lines (lane l: lines y0 + l + 32 t); per entry (j, v) of a row it reads the entry once and one coalesced
-// 128-byte segment of column j per 32 lines, four entries in flight, paired fused multiply-adds. A block's 8 warps
+// 32 ZT_G lines (ZtLines); per entry (j, v) of a row it reads the entry once and column j's lines in 512-byte
+// segments, several entries in flight, paired fused multiply-adds. L2 bounds it (76 % of its peak at 288 lines: every
+// entry reads a column from there). With a guarded 4-byte load per 32 lines, 43 instructions per entry, the 360
+// angles of 256 x 256 pixels, 1012 channels took 3.94 ms (transposes in), now 3.38; 180 of 99 x 99 0.83, now 0.59. A block's 8 warps
 // hold 8 kw consecutive orientations, written as whole row segments of the Radon input through shared memory (kw is
 // the largest that still gives the launch a few waves of blocks). Per output the sum runs over the row's entries in
 // order with fmaf from 0 and is scaled by alpha: spmm_adjoint8_kernel's bits.
 constexpr int AZ_KW = 4;                 // orientation rows per warp at most
 constexpr int AZ_WARPS = 8;
 
-// dt[s][j][y] = data[r(s)][y][j] (j < cp, y < my; zero for my <= y < ly), r(s) = omegas[s] or r0 + s
-__global__ void __launch_bounds__(256) dt_transpose_kernel(const float *__restrict__ data, float *__restrict__ dt,
-                                                           const int32_t *__restrict__ omegas, int r0, int my, int ly,
-                                                           int cp)
-{
-    __shared__ float tile[ZT_TR][ZT_TR + 1];
-    const int s = blockIdx.z, j0 = blockIdx.x * ZT_TR, y0 = blockIdx.y * ZT_TR;
-    const int r = omegas ? __ldg(omegas + s) : r0 + s;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    for (int yy = ty; yy < ZT_TR; yy += 8) {
-        const int y = y0 + yy, j = j0 + tx;
-        tile[yy][tx] = (y < my && j < cp) ? __ldg(data + ((int64_t)r * my + y) * cp + j) : 0.0f;
-    }
-    __syncthreads();
-    for (int jj = ty; jj < ZT_TR; jj += 8) {
-        const int j = j0 + jj;
-        if (j < cp) dt[((int64_t)s * cp + j) * ly + y0 + tx] = tile[tx][jj];
-    }
-}
-
 template <int MT>
-__global__ void __launch_bounds__(32 * AZ_WARPS, 3) spmm_adjoint_zt_kernel(
+__global__ void __launch_bounds__(32 * AZ_WARPS, MT > 6 ? 3 : 4) spmm_adjoint_zt_kernel(
     const float *__restrict__ dt, const int32_t *__restrict__ row_ptr, const uint16_t *__restrict__ col_j,
     const float *__restrict__ val, float *__restrict__ sino, const int32_t *__restrict__ omegas, int r0, int my,
     int ly, int kb, int cp, int kstride, float alpha, int compact, int kw)
 {
+    constexpr int U = zt_ua(MT);
     extern __shared__ float s_outk[];                 // [32 MT][8 kw + 1]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int s = blockIdx.z;
     const int r = omegas ? __ldg(omegas + s) : r0 + s;
     const int ngroups = ly >> 5;
-    const int g0 = blockIdx.y * MT;
-    const int y0 = g0 * 32;
+    const int g0 = min((int)blockIdx.y * MT, ngroups - MT);    // as in spmm_forward_zt_kernel
+    const int y0 = g0 * 32, yskip = ((int)blockIdx.y * MT - g0) * 32;
     const int nk = AZ_WARPS * kw, ldk = nk + 1;
     const int k0 = blockIdx.x * nk;
-    const float *ds = dt + (int64_t)s * cp * ly + y0 + lane;
+    const ZtLines<MT> zl(dt + (int64_t)s * cp * ly + y0, lane);
+    const uint32_t col_b = (uint32_t)ly * 4u;
+    // a lane's row pointer: rows k0 + warp kw .. + kw of the angle (rows past kb are empty)
+    const int64_t rr = (int64_t)(compact ? s : r) * kb;
+    const int ptr = __ldg(row_ptr + rr + min(k0 + warp * kw + min(lane, kw), kb));
     for (int kk = 0; kk < kw; ++kk) {
         const int kl = warp * kw + kk, k = k0 + kl;
-        int i = 0, e = 0;
-        if (k < kb) {
-            const int64_t rr = (int64_t)(compact ? s : r) * kb + k;
-            i = __ldg(row_ptr + rr);
-            e = __ldg(row_ptr + rr + 1);
-        }
+        int i = __shfl_sync(0xffffffffu, ptr, kk);
+        const int e = __shfl_sync(0xffffffffu, ptr, kk + 1);
         float acc[MT];
 #pragma unroll
         for (int t = 0; t < MT; ++t) acc[t] = 0.0f;
-        int jq[ZT_U];
-        float vq[ZT_U];
+        uint32_t jq[U];
+        float vq[U];
+        if (i + U <= e) {
 #pragma unroll
-        for (int q = 0; q < ZT_U; ++q) {
-            jq[q] = i + q < e ? __ldg(col_j + i + q) : 0;
-            vq[q] = i + q < e ? __ldg(val + i + q) : 0.0f;
+            for (int q = 0; q < U; ++q) {
+                jq[q] = __ldg(col_j + i + q);
+                vq[q] = __ldg(val + i + q);
+            }
         }
-        for (; i < e; i += ZT_U) {
-            float vc[ZT_U];
-            float z[ZT_U][MT];
+        for (; i + U <= e; i += U) {
+            float vc[U];
+            float z[U][MT];
 #pragma unroll
-            for (int q = 0; q < ZT_U; ++q) {
+            for (int q = 0; q < U; ++q) {
                 vc[q] = vq[q];
-                const float *zc = ds + (int64_t)jq[q] * ly;
-#pragma unroll
-                for (int t = 0; t < MT; ++t) z[q][t] = g0 + t < ngroups ? __ldg(zc + 32 * t) : 0.0f;
+                zl.load(jq[q] * col_b, z[q]);
             }
 #pragma unroll
-            for (int q = 0; q < ZT_U; ++q) {
-                jq[q] = i + ZT_U + q < e ? __ldg(col_j + i + ZT_U + q) : 0;
-                vq[q] = i + ZT_U + q < e ? __ldg(val + i + ZT_U + q) : 0.0f;
+            for (int q = 0; q < U; ++q) {
+                const int f = min(i + U + q, e - 1);
+                jq[q] = __ldg(col_j + f);
+                vq[q] = __ldg(val + f);
             }
 #pragma unroll
-            for (int q = 0; q < ZT_U; ++q) {
-                if (i + q < e) {
-#pragma unroll
-                    for (int t = 0; t + 1 < MT; t += 2) fma_pair(acc[t], acc[t + 1], vc[q], z[q][t], z[q][t + 1]);
-                    if (MT & 1) acc[MT - 1] = __fmaf_rn(vc[q], z[q][MT - 1], acc[MT - 1]);
-                }
-            }
+            for (int q = 0; q < U; ++q) fma_lines<MT>(acc, vc[q], z[q]);
+        }
+        for (; i < e; ++i) {
+            float z[MT];
+            zl.load(__ldg(col_j + i) * col_b, z);
+            fma_lines<MT>(acc, __ldg(val + i), z);
         }
 #pragma unroll
         for (int t = 0; t < MT; ++t) s_outk[(lane + 32 * t) * ldk + kl] = k < kb ? alpha * acc[t] : 0.0f;
@@ -691,8 +717,9 @@ __global__ void __launch_bounds__(32 * AZ_WARPS, 3) spmm_adjoint_zt_kernel(
     const int kl = threadIdx.x % nk, ty = threadIdx.x / nk;
     const int k = k0 + kl;
     if (k < kstride) {
-        float *zl = sino + ((int64_t)s * my + y0) * kstride + k;
-        for (int yl = ty; yl < ny; yl += (32 * AZ_WARPS) / nk) zl[(int64_t)yl * kstride] = s_outk[yl * ldk + kl];
+        float *out = sino + ((int64_t)s * my + y0) * kstride + k;
+        for (int yl = yskip + ty; yl < ny; yl += (32 * AZ_WARPS) / nk)
+            out[(int64_t)yl * kstride] = s_outk[ZtLines<MT>::slot(yl) * ldk + kl];
     }
 }
 
@@ -788,12 +815,12 @@ extern "C" int64_t dfx_spmm_pf_forward_zt_floats(int n_angles, int my, int kb)
     return (int64_t)n_angles * kb * (cdiv(my, 32) * 32);
 }
 
-template <int MT>
-static int launch_zt(const float *zt, const int32_t *fb_ptr, const uint16_t *fb_k, const float *fb_v,
-                     const uint8_t *fb_mask, float *data, const int32_t *omegas, int r0, int na, int my, int ly,
-                     int nyb, int P, int C, int ncb, int nb, int kb, cudaStream_t st)
+template <int MT, bool WIDE>
+static int launch_zt_as(const float *zt, const int32_t *fb_ptr, const uint16_t *fb_k, const float *fb_v,
+                        const uint8_t *fb_mask, float *data, const int32_t *omegas, int r0, int na, int my, int ly,
+                        int nyb, int P, int C, int ncb, int nb, int kb, cudaStream_t st)
 {
-    const cudaError_t err = allow_max_dynamic_smem(spmm_forward_zt_kernel<MT>);
+    const cudaError_t err = allow_max_dynamic_smem(spmm_forward_zt_kernel<MT, WIDE>);
     if (err != cudaSuccess) {
         set_error("spmm_forward_blocked_zt: shared memory attribute: %s", cudaGetErrorString(err));
         return DFX_ELAUNCH;
@@ -801,9 +828,30 @@ static int launch_zt(const float *zt, const int32_t *fb_ptr, const uint16_t *fb_
     const int width = FB_W * nb * P;
     const size_t smem = (size_t)32 * MT * (width + 1) * sizeof(float);
     dim3 grid((unsigned)cdiv(ncb, nb), (unsigned)nyb, (unsigned)na);
-    spmm_forward_zt_kernel<MT><<<grid, 256, smem, st>>>(zt, fb_ptr, fb_k, reinterpret_cast<const float4 *>(fb_v),
-                                                        fb_mask, data, omegas, r0, my, ly, P, C, ncb, nb, kb);
+    spmm_forward_zt_kernel<MT, WIDE><<<grid, 32 * std::min(8, nb * P), smem, st>>>(
+        zt, fb_ptr, fb_k, reinterpret_cast<const float4 *>(fb_v), fb_mask, data, omegas, r0, my, ly, P, C, ncb, nb, kb);
     return launch_status("spmm_pf_forward_blocked_zt");
+}
+
+template <int MT>
+static int launch_zt(const float *zt, const int32_t *fb_ptr, const uint16_t *fb_k, const float *fb_v,
+                     const uint8_t *fb_mask, float *data, const int32_t *omegas, int r0, int na, int my, int ly,
+                     int nyb, int P, int C, int ncb, int nb, int kb, cudaStream_t st)
+{
+    int dev = 0, nsm = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    // fewer blocks than SMs: fewer eta blocks each (12 angles of 90 eta bins x 3 rings, 53 lines: 60 blocks of 15 rows
+    // 44 us, 276 of 3 rows 28 us; at 18 angles of 180 x 5, 103 lines, 270 blocks of 15 rows are the faster ones, 69
+    // against 87 us with 5 rows: the rows are taken longest first and the write-back has whole segments)
+    while (nb > 1 && cdiv(ncb, nb) * nyb * na < nsm) --nb;
+    // from four waves on three blocks of 80 registers per SM with three entries in flight per warp are the faster ones
+    // (360 angles at 256 x 256 pixels, 1012 channels, both transposes in: 1.86 against 2.05 ms; 180 at 99 x 99: 0.56
+    // against 0.63), below two of 128 with four entries (18 angles at 99 x 99: 69 against 74 us)
+    if (MT > 2 && cdiv(ncb, nb) * nyb * na >= 4LL * 3 * nsm)
+        return launch_zt_as<MT, true>(zt, fb_ptr, fb_k, fb_v, fb_mask, data, omegas, r0, na, my, ly, nyb, P, C, ncb, nb,
+                                      kb, st);
+    return launch_zt_as<MT, false>(zt, fb_ptr, fb_k, fb_v, fb_mask, data, omegas, r0, na, my, ly, nyb, P, C, ncb, nb, kb,
+                                   st);
 }
 
 extern "C" int dfx_spmm_pf_forward_blocked_zt(const float *sino, float *zt, int64_t zt_floats, const int32_t *fb_ptr,
@@ -818,21 +866,25 @@ extern "C" int dfx_spmm_pf_forward_blocked_zt(const float *sino, float *zt, int6
     DFX_REQUIRE(P <= 32, "spmm_forward_blocked_zt: more than 32 rings");
     const int64_t per_angle = dfx_spmm_pf_forward_zt_floats(1, my, kb);
     DFX_REQUIRE(zt_floats >= per_angle, "spmm_forward_blocked_zt: the transpose buffer holds less than one angle");
-    const int ly = (int)(cdiv(my, 32) * 32), ngroups = ly / 32;
     DFX_REQUIRE(max_groups >= 0 && max_groups <= ZT_G, "spmm_forward_blocked_zt: max_groups outside 0 .. 9");
+    // the lines are read 16 bytes at a time at 32-bit byte offsets in an angle: otherwise the same sums without a buffer
+    if ((uintptr_t)zt % 16 != 0 || per_angle * 4 >= ((int64_t)1 << 32))
+        return dfx_spmm_pf_forward_blocked(sino, fb_ptr, fb_k, fb_v, fb_mask, data, omegas, n_sub, my, P, C, kstride, kb,
+                                           stream);
+    const int ly = (int)(cdiv(my, 32) * 32), ngroups = ly / 32;
     const int gmax = max_groups ? max_groups : ZT_G;
     const int nyb = (int)cdiv(ngroups, gmax), mt = (int)cdiv(ngroups, nyb);
     // blocks of nb eta blocks x all rings: at most 16 rows (one eta block above 16 rings)
     const int nb = P >= 16 ? 1 : 16 / P;
     const int ncb = (int)cdiv(C, FB_W);
-    DFX_REQUIRE(nyb <= 65535 && cdiv(kb, ZT_TR) <= 2147483647LL, "spmm_forward_blocked_zt: grid too large");
+    DFX_REQUIRE(nyb <= 65535 && kb <= 65536, "spmm_forward_blocked_zt: grid too large");
     const int chunk = (int)std::min<int64_t>(std::min<int64_t>(n_sub, zt_floats / per_angle), 65535);
     cudaStream_t st = (cudaStream_t)stream;
     for (int s0 = 0; s0 < n_sub; s0 += chunk) {
         const int na = std::min(chunk, n_sub - s0);
-        dim3 tg((unsigned)cdiv(kb, ZT_TR), (unsigned)(ly / ZT_TR), (unsigned)na);
-        zt_transpose_kernel<<<tg, 256, 0, st>>>(sino + (int64_t)s0 * my * kstride, zt, my, ly, kstride, kb);
-        int rc = launch_status("spmm_pf_forward_blocked_zt: transpose");
+        // zt[s][k][y] = sino[s][y][k] (k < kb, y < my; zero for my <= y < ly)
+        int rc = launch_transpose(sino + (int64_t)s0 * my * kstride, kstride, (int64_t)my * kstride, nullptr, 0, zt, ly,
+                                  (int64_t)kb * ly, my, ly, kb, na, st);
         if (rc) return rc;
         const int32_t *om = omegas ? omegas + s0 : nullptr;
         switch (mt) {
@@ -899,6 +951,9 @@ extern "C" int dfx_spmm_pf_adjoint_zt(const float *data, float *dt, int64_t dt_f
     DFX_REQUIRE(max_groups >= 0 && max_groups <= ZT_G, "spmm_adjoint_zt: max_groups outside 0 .. 9");
     const int64_t per_angle = dfx_spmm_pf_adjoint_zt_floats(1, my, cp);
     DFX_REQUIRE(dt_floats >= per_angle, "spmm_adjoint_zt: the transpose buffer holds less than one angle");
+    if ((uintptr_t)dt % 16 != 0 || per_angle * 4 >= ((int64_t)1 << 32))     // as the forward's
+        return dfx_spmm_pf_adjoint(data, row_ptr, col_j, val, sino, omegas, n_sub, my, kb, cp, kstride, alpha, compact,
+                                   stream);
     const int ly = (int)(cdiv(my, 32) * 32), ngroups = ly / 32;
     const int gmax = max_groups ? max_groups : ZT_G;
     const int nyb = (int)cdiv(ngroups, gmax), mt = (int)cdiv(ngroups, nyb);
@@ -908,9 +963,8 @@ extern "C" int dfx_spmm_pf_adjoint_zt(const float *data, float *dt, int64_t dt_f
     for (int s0 = 0; s0 < n_sub; s0 += chunk) {
         const int na = std::min(chunk, n_sub - s0);
         const int32_t *om = omegas ? omegas + s0 : nullptr;
-        dim3 tg((unsigned)cdiv(cp, ZT_TR), (unsigned)(ly / ZT_TR), (unsigned)na);
-        dt_transpose_kernel<<<tg, 256, 0, st>>>(data, dt, om, s0, my, ly, cp);
-        int rc = launch_status("spmm_pf_adjoint_zt: transpose");
+        // dt[s][j][y] = data[r(s)][y][j] (j < cp, y < my; zero for my <= y < ly), r(s) = omegas[s] or s0 + s
+        int rc = launch_transpose(data, cp, (int64_t)my * cp, om, s0, dt, ly, (int64_t)cp * ly, my, ly, cp, na, st);
         if (rc) return rc;
         // compact rows are numbered by the position in the subset: the chunk's rows start at s0 * kb
         const int32_t *rp = compact ? row_ptr + (int64_t)s0 * kb : row_ptr;

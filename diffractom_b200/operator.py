@@ -64,8 +64,8 @@ class SinglePhaseForwardOperator:
     # whole 128-byte segments of a data column per entry; dfx_spmm_pf_adjoint_zt, the same bits) through the same
     # buffer; False: dfx_spmm_pf_adjoint on the segment-fastest rows
     adjoint_lines_fastest = True
-    zt_max_angles = 64                   # angles per transpose chunk at most
-    zt_max_bytes = 256 * 1024 ** 2       # the transpose buffer at most (at least one angle)
+    zt_max_angles = 256                  # angles per transpose chunk at most
+    zt_max_bytes = 512 * 1024 ** 2       # the transpose buffer at most (at least one angle)
     zt_max_groups = 0
 
     def __init__(self, cfg: Mapping[str, Any], material, grid, max_gb: float, verbose: bool = False,
