@@ -769,25 +769,36 @@ __global__ void __launch_bounds__(32 * BW, 6) radon_backward_tile(
 // mode 0: x = 1 inside the support on live channels, else 0 (support_ones); mode 1: x = 0 outside the support, on
 // padding channels or where negative (project_support); mode 2: T = min(T, c / colsum) inside the support where
 // colsum > 0 (tmin).
-__global__ void batch_support_kernel(float *__restrict__ x, const float *__restrict__ colsum,
-                                     const uint8_t *__restrict__ supp, int64_t npix, int kstride, int kb, float c,
-                                     int mode)
+// V channels per step (4 where the stride and the arrays allow 16-byte accesses), with 32-bit indices where they reach.
+// HBM bounds it: on 256 x 256 pixels x 960 channels 0.23 ms with one channel per step and 64-bit divisions, now 0.11.
+template <int V, typename Index>
+__global__ void __launch_bounds__(256) batch_support_kernel(float *__restrict__ x, const float *__restrict__ colsum,
+                                                            const uint8_t *__restrict__ supp, int64_t npix, int kstride,
+                                                            int kb, float c, int mode)
 {
-    const int64_t n = npix * kstride;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t p = i / kstride;
-        const int k = (int)(i - p * kstride);
-        const bool inside = (supp ? __ldg(supp + p) != 0 : true) && k < kb;
-        if (mode == 0) {
-            x[i] = inside ? 1.0f : 0.0f;
-        } else if (mode == 1) {
-            if (!inside || x[i] < 0.0f) x[i] = 0.0f;
-        } else if (mode == 3) {
-            if (!inside) x[i] = 0.0f;
+    const Index kv = (Index)(kstride / V), n = (Index)npix * kv;
+    for (Index i = blockIdx.x * (Index)256 + threadIdx.x; i < n; i += (Index)gridDim.x * 256) {
+        const Index p = i / kv;
+        const int k = (int)(i - p * kv) * V;
+        const bool in = supp ? __ldg(supp + p) != 0 : true;
+        alignas(16) float r[V], cs[V];
+        if (V == 4) {
+            if (mode != 0) *reinterpret_cast<float4 *>(r) = reinterpret_cast<const float4 *>(x)[i];
+            if (mode == 2) *reinterpret_cast<float4 *>(cs) = __ldg(reinterpret_cast<const float4 *>(colsum) + i);
         } else {
-            const float cs = colsum[i];
-            if (inside && cs > 0.0f) x[i] = fminf(x[i], __fdiv_rn(c, cs));
+            if (mode != 0) r[0] = x[i];
+            if (mode == 2) cs[0] = __ldg(colsum + i);
         }
+#pragma unroll
+        for (int q = 0; q < V; ++q) {
+            const bool inside = in && k + q < kb;
+            if (mode == 0) r[q] = inside ? 1.0f : 0.0f;
+            else if (mode == 1) r[q] = !inside || r[q] < 0.0f ? 0.0f : r[q];
+            else if (mode == 3) r[q] = inside ? r[q] : 0.0f;
+            else if (inside && cs[q] > 0.0f) r[q] = fminf(r[q], __fdiv_rn(c, cs[q]));
+        }
+        if (V == 4) reinterpret_cast<float4 *>(x)[i] = *reinterpret_cast<const float4 *>(r);
+        else x[i] = r[0];
     }
 }
 
@@ -1144,8 +1155,12 @@ extern "C" int dfx_batch_support(float *x_k, const float *colsum_k, const uint8_
     DFX_REQUIRE(x_k && npix > 0 && kstride > 0 && kb >= 0 && kb <= kstride && mode >= 0 && mode <= 3,
                 "batch_support: bad arguments");
     DFX_REQUIRE(mode != 2 || colsum_k, "batch_support: tmin needs the column sums");
-    const int64_t blocks = cdiv(npix * kstride, 256);
-    batch_support_kernel<<<(unsigned)(blocks < 148 * 32 ? blocks : 148 * 32), 256, 0, (cudaStream_t)stream>>>(
+    const bool vec = kstride % 4 == 0 && (uintptr_t)x_k % 16 == 0 && (mode != 2 || (uintptr_t)colsum_k % 16 == 0);
+    const int64_t n = npix * (vec ? kstride / 4 : kstride), blocks = cdiv(n, 256);
+    const bool small = n < ((int64_t)1 << 31);
+    const auto kernel = vec ? (small ? batch_support_kernel<4, uint32_t> : batch_support_kernel<4, int64_t>)
+                            : (small ? batch_support_kernel<1, uint32_t> : batch_support_kernel<1, int64_t>);
+    kernel<<<(unsigned)(blocks < 148 * 32 ? blocks : 148 * 32), 256, 0, (cudaStream_t)stream>>>(
         x_k, colsum_k, supp, npix, kstride, kb, c, mode);
     return launch_status("batch_support");
 }
