@@ -36,7 +36,7 @@ AUTO_FFT_PIXELS = 400 * 400   # projector="auto": the Fourier-slice projector fo
 SPARSE_MIN_BATCHES = 4    # sparse modes: at least this many batches (SPFO:135)
 CAND_BYTES = 2 + 4 + 4 + 4 + 4          # per candidate / non-zero scratch of the reference's generator
 NNZ_BYTES = 2 + 4 + 4 + 2 + 4 + 2 + 4   # (pf_generate.py:29-30), used by the batch-size rule
-GTABLE_MIN_WARPS = 4 * 148 * 32          # forwards of a scan with this many grouped-table warps read the grouped table
+GTABLE_MIN_WARPS = 3 * 148 * 32          # forwards of a scan with this many grouped-table warps read the grouped table
 KSTRIDE_ALIGN = 16                       # channel stride of the batch buffers (16 channels per tensor-memory load)
 
 
@@ -383,8 +383,8 @@ class SinglePhaseForwardOperator:
         grp = self._ray_grp if ray is None else (ray[3] if len(ray) > 3 else None)
         # a scan's consecutive angles share their pixels in L1 through the grouped table, a subset's do not (18 angles
         # at 256 x 256 pixels, 1012 channels: 0.75 ms grouped, 0.44 ms per-bin; all 360: 6.6 and 7.2 ms). It has a
-        # quarter of the warps: below about four waves of them the per-bin table is as fast (180 angles of 99 x 99
-        # pixels, 4 waves: 0.556 and 0.560 ms) or faster (91 angles of 131 x 131 pixels, 333 channels, 1.3 waves: 0.31
+        # quarter of the warps: below about three waves of them the per-bin table is the faster one (180 angles of 99
+        # x 99 pixels, 4 waves: 0.53 grouped, 0.56 ms per-bin; 91 of 131 x 131 pixels, 333 channels, 1.3 waves: 0.31
         # and 0.26 ms; 90 of 48 x 48, half a wave: 0.069 and 0.048 ms)
         warps = n_ang * -(-self.My // 4) * -(-self.Kstride // 256)
         if grp is not None and m is None and warps >= GTABLE_MIN_WARPS:

@@ -151,6 +151,12 @@ class SPDHGPoisson:
         return [-1 if i in tv_at else next(it) for i in range(n)]
 
     # ---------------------------------------------------------------- device steps
+    def _zero_next(self, m):
+        """D's rows of subset m = 0 before a pass adds its forward batch by batch; a BF16 operator's pass overwrites
+        them with one product over all batches."""
+        if self.op.precision != "bf16":
+            self.op.zero_subset_rows(self.D, m)
+
     def _dual(self, m):
         op = self.op
         e = op._sub[m]
@@ -719,7 +725,7 @@ class SPDHGPoisson:
             else:
                 self.xkb = torch.empty(be, dtype=torch.bfloat16, device=dev)
         if self._seq[0] >= 0:
-            op.zero_subset_rows(self.D, self._seq[0])
+            self._zero_next(self._seq[0])
             self._pass(None, self._seq[0])
 
     @on_op_stream
@@ -762,7 +768,7 @@ class SPDHGPoisson:
                     # this epoch's residual on the side stream; the next subset's rows by the usual pass
                     if adj is not None:
                         self._dual(adj)
-                    op.zero_subset_rows(self.D, m_next)
+                    self._zero_next(m_next)
                     self._pass(adj, m_next, tv=tvb)
                     self._residual_async(len(self.iter_stats))
                     continue
@@ -782,11 +788,10 @@ class SPDHGPoisson:
                                 self._f += self.tv * self._tv_value()
                 elif graphed:
                     self._replay(("update", adj), lambda m=adj: (self._dual(m), self._pass(m, None)))
-                    self._replay(("forward", m_next), lambda nb=m_next: (op.zero_subset_rows(self.D, nb),
-                                                                         self._pass(None, nb)))
+                    self._replay(("forward", m_next), lambda nb=m_next: (self._zero_next(nb), self._pass(None, nb)))
                 else:
                     if m_next is not None:
-                        op.zero_subset_rows(self.D, m_next)
+                        self._zero_next(m_next)
                     self._pass(adj, m_next, tv=tvb)
             if nseq is not None:
                 seq = nseq

@@ -97,3 +97,23 @@ def test_reflection_two_theta_geometry_matches_reference(golden):
     assert np.array_equal(g.axis_start_cpu, d["start"]) and np.allclose(g.pole_axes_cpu, d["axes"], atol=1e-12)
     assert np.allclose(g.axis_two_theta_cpu, d["axis_two_theta"], rtol=0, atol=1e-14)
     assert len(np.unique(np.round(g.axis_two_theta_cpu[d["start"][0]:d["start"][1]], 9))) == 2   # two angles in a window
+
+
+def test_fov_support_mask_equals_every_pixel_at_every_angle():
+    """The mask tried on the pixels outside the inner disk only = every pixel tried at every angle, also with the edge on
+    pixel centres (angles of 0, 45, 90 degrees, half-integer detectors), shifts, and detectors smaller than a pixel."""
+    from diffractom_b200.geometry import fov_support_mask
+    rng = np.random.default_rng(0)
+    for _ in range(200):
+        nx, ny, nd, R = (int(v) for v in rng.integers(1, [70, 70, 90, 40]))
+        ang = np.deg2rad(rng.choice([0.0, 0.25, 17.3]) + np.arange(R) * rng.choice([1, 2, 4.5, 15, 45, 90]))
+        shift, width = rng.choice([0, 0.5, -3.25, 100.0]), rng.choice([1.0, 0.5, 1.7]) * max(nx, ny)
+        dx = width / max(nx, ny)
+        x = (np.arange(nx) - (nx - 1) / 2.0)[None, :] * dx
+        y = (np.arange(ny) - (ny - 1) / 2.0)[:, None] * dx
+        want = np.ones((ny, nx), bool)
+        for a in ang:
+            t = np.cos(a - 0.5 * np.pi) * x + np.sin(a - 0.5 * np.pi) * y - shift
+            want &= np.abs(t) <= nd / 2.0 + 1e-9 * nd
+        got = fov_support_mask(nx, ny, nd, angles=ang, image_width=width, detector_width=nd, detector_shift=shift)
+        assert np.array_equal(got, want)
