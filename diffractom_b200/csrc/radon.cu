@@ -835,6 +835,8 @@ static int launch_backward(const ST *sino, int64_t sld, float *img, const float 
                            __nv_bfloat16 *xb, void *stream, const int32_t *plist = nullptr, int64_t n_list = 0)
 {
     const int64_t npix = plist ? n_list : (int64_t)nx * ny;
+    const size_t smem = sizeof(AngleParams) * (size_t)(n_angles > 0 ? n_angles : 1);
+    DFX_REQUIRE(smem <= 200 * 1024, "radon: %d angles exceed the shared memory of one launch", n_angles);
     // pixels with at most two taps, an angle's rows within 32-bit byte offsets: neighbouring pixels share their bins
     if (!plist && n_taps == 2 && (int64_t)n_det * sld * (int64_t)sizeof(ST) < ((int64_t)1 << 32)) {
         const dim3 tiles((unsigned)(cdiv(nx, TX) * cdiv(ny, BW)), (unsigned)cdiv(kstride, CPW));
@@ -850,8 +852,6 @@ static int launch_backward(const ST *sino, int64_t sld, float *img, const float 
     const bool pair = kstride > CPW;
     dim3 grid((unsigned)cdiv(npix, WARPS), (unsigned)cdiv(kstride, pair ? 2 * CPW : CPW));
     DFX_REQUIRE(grid.x < 2147483647u && grid.y <= 65535u, "radon: batch too large for one launch");
-    const size_t smem = sizeof(AngleParams) * (size_t)(n_angles > 0 ? n_angles : 1);
-    DFX_REQUIRE(smem <= 200 * 1024, "radon: %d angles exceed the shared memory of one launch", n_angles);
     int st = pair ? allow_smem(radon_backward_v3<KERNEL, MODE, ST, 2>, smem)
                   : allow_smem(radon_backward_v3<KERNEL, MODE, ST, 1>, smem);
     if (st) return st;

@@ -877,7 +877,7 @@ extern "C" int dfx_spmm_pf_forward_blocked_zt(const float *sino, float *zt, int6
     // blocks of nb eta blocks x all rings: at most 16 rows (one eta block above 16 rings)
     const int nb = P >= 16 ? 1 : 16 / P;
     const int ncb = (int)cdiv(C, FB_W);
-    DFX_REQUIRE(nyb <= 65535 && kb <= 65536, "spmm_forward_blocked_zt: grid too large");
+    DFX_REQUIRE(nyb <= 65535, "spmm_forward_blocked_zt: grid too large");
     const int chunk = (int)std::min<int64_t>(std::min<int64_t>(n_sub, zt_floats / per_angle), 65535);
     cudaStream_t st = (cudaStream_t)stream;
     for (int s0 = 0; s0 < n_sub; s0 += chunk) {
