@@ -20,19 +20,13 @@
 #include <tuple>
 
 #include "dfx_common.cuh"
+#include "fourier_taps.cuh"
 
 namespace dfx {
 namespace {
 
-constexpr int FR_TS = 16;     // spreading tile (cells per side)
 constexpr int FR_SB = 64;     // samples staged per round of the spread
 constexpr int FR_CCS = 16;    // channels per spreading block
-
-__device__ __forceinline__ int wrap(int v, int m)
-{
-    int r = v % m;
-    return r < 0 ? r + m : r;
-}
 
 // image slice (channel-fastest, channels c0 .. c0+cb-1 of img_k) -> grid (C, My, Mx); a block: 32 grid columns x 32
 // channels of one grid row
@@ -177,7 +171,8 @@ __global__ void __launch_bounds__(FR_TS *FR_TS) fr_spread_kernel(
     const int tile = pc.x, cg = blockIdx.y * FR_CCS;
     const int lx = threadIdx.x, ly = threadIdx.y, lid = ly * FR_TS + lx;
     const int Hx = Mx / 2 + 1;
-    const int q1 = (tile % n_tx) * FR_TS + lx, q2 = (tile / n_tx) * FR_TS + ly;
+    // the thread's cell; threads past the half grid (FR_OFF) have no taps
+    const int q1 = fr_cell((tile % n_tx) * FR_TS + lx, Hx), q2 = fr_cell((tile / n_tx) * FR_TS + ly, My);
     float2 acc[FR_CCS];
 #pragma unroll
     for (int c = 0; c < FR_CCS; ++c) acc[c] = make_float2(0.0f, 0.0f);
@@ -190,8 +185,8 @@ __global__ void __launch_bounds__(FR_TS *FR_TS) fr_spread_kernel(
             const bool mir = sm < 0;
             const int2 b = __ldg(kb + smp);
             lmir[lid] = mir;
-            lb1[lid] = wrap(mir ? -b.x : b.x, Mx);                // tap offset d = q - b, or b - q through the mirror
-            lb2[lid] = wrap(mir ? -b.y : b.y, My);
+            lb1[lid] = fr_first(b.x, mir, Mx);
+            lb2[lid] = fr_first(b.y, mir, My);
             const int j = smp % H;
             lhalf[lid] = (j == 0 || j == H - 1) ? 0.5f : 1.0f;
 #pragma unroll
@@ -209,22 +204,15 @@ __global__ void __launch_bounds__(FR_TS *FR_TS) fr_spread_kernel(
         // a warp holds two rows of the tile: of 32 samples at a time, those with a tap on one of the rows (a ballot
         // instead of a try per thread, and two channels per shared load: 1.30 -> 1.08 ms per slice of 128 channels at 416 x
         // 416 pixels and 360 angles; broadcasts of the staged values bound it)
-        const int row0 = (tile / n_tx) * FR_TS + (ly & ~1);
+        const int row0 = fr_cell((tile / n_tx) * FR_TS + (ly & ~1), My);
         for (int h = 0; h < nb; h += 32) {
             const int u = h + (lid & 31);
-            bool near = false;
-            if (u < nb) {
-                const int e = lmir[u] ? lb2[u] - row0 : row0 - lb2[u], f = lmir[u] ? e - 1 : e + 1;
-                near = (e < 0 ? e + My : e) < W || (f < 0 ? f + My : f) < W;
-            }
+            const bool near = u < nb && fr_rows_near(row0, lb2[u], lmir[u] != 0, My, W);
             for (uint32_t left = __ballot_sync(0xFFFFFFFFu, near); left; left &= left - 1) {
                 const int t = h + __ffs(left) - 1;
                 const bool mir = lmir[t] != 0;
-                int d1 = mir ? lb1[t] - q1 : q1 - lb1[t];
-                int d2 = mir ? lb2[t] - q2 : q2 - lb2[t];
-                d1 += d1 < 0 ? Mx : 0;
-                d2 += d2 < 0 ? My : 0;
-                if (d1 < W && d2 < W) {
+                int d1, d2;
+                if (fr_tap(q1, lb1[t], mir, Mx, W, d1) && fr_tap(q2, lb2[t], mir, My, W, d2)) {
                     const float w = __fmul_rn(__fmul_rn(lw2[t][d2], lw1[t][d1]), lhalf[t]), wi = mir ? -w : w;
 #pragma unroll
                     for (int c = 0; c < FR_CCS; c += 2) {
@@ -238,7 +226,7 @@ __global__ void __launch_bounds__(FR_TS *FR_TS) fr_spread_kernel(
             }
         }
     }
-    if (q1 < Hx && q2 < My) {
+    if (q1 != FR_OFF && q2 != FR_OFF) {
 #pragma unroll
         for (int c = 0; c < FR_CCS; ++c) {
             if (cg + c >= C) break;

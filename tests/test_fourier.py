@@ -2,6 +2,10 @@
 interpolation, 1-D inverse FFT; and the transposed steps with the spreading tile lists) built from the same float32
 tables matches the exact Fourier-slice projection of the oracle to the NUFFT's accuracy, and the exact projection
 agrees with the native (hat) projector to the few per cent that separate the two projectors."""
+import ctypes
+import subprocess
+from pathlib import Path
+
 import numpy as np
 import pytest
 
@@ -135,3 +139,67 @@ def test_spreading_pieces_partition_every_tile_list():
         assert np.array_equal(mine[1:, 1], mine[:-1, 2]) and np.all(mine[:, 2] - mine[:, 1] <= PIECE)
         assert mine[0, 3] == -1 and np.array_equal(mine[1:, 3], np.arange(tab.tile_xptr[t], tab.tile_xptr[t + 1]))
     assert tab.n_slots == len(pc) - tab.n_tiles
+
+
+REPLAY = r"""
+#include "fourier_taps.cuh"
+#include <cstdint>
+using namespace dfx;
+// out[entry][thread] = d2 W + d1 of the tap that the spread's thread applies for the tile list's entry, -1: none
+extern "C" void replay(const int32_t *tile_ptr, const int32_t *tile_smp, const int32_t *kb, int n_tiles, int n_tx,
+                       int Mx, int My, int W, int32_t *out)
+{
+    for (int tile = 0; tile < n_tiles; ++tile)
+        for (int e = tile_ptr[tile]; e < tile_ptr[tile + 1]; ++e) {
+            const int sm = tile_smp[e], smp = sm >= 0 ? sm : -sm - 1;
+            const bool mir = sm < 0;
+            const int b1 = fr_first(kb[2 * smp], mir, Mx), b2 = fr_first(kb[2 * smp + 1], mir, My);
+            for (int lid = 0; lid < FR_TS * FR_TS; ++lid) {
+                const int lx = lid % FR_TS, ly = lid / FR_TS;
+                const int q1 = fr_cell(tile % n_tx * FR_TS + lx, Mx / 2 + 1), q2 = fr_cell(tile / n_tx * FR_TS + ly, My);
+                int d1, d2, &o = out[(int64_t)e * FR_TS * FR_TS + lid] = -1;
+                if (!fr_rows_near(fr_cell(tile / n_tx * FR_TS + (ly & ~1), My), b2, mir, My, W)) continue;
+                if (fr_tap(q1, b1, mir, Mx, W, d1) && fr_tap(q2, b2, mir, My, W, d2))
+                    o = d1 >= 0 && d2 >= 0 && d1 < W && d2 < W ? d2 * W + d1 : -2;
+            }
+        }
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def replay(tmp_path_factory):
+    """The spread's index arithmetic (csrc/fourier_taps.cuh) compiled for the host."""
+    d = tmp_path_factory.mktemp("replay")
+    (d / "replay.cpp").write_text(REPLAY)
+    inc = Path(__file__).resolve().parents[1] / "diffractom_b200" / "csrc"
+    subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-I", str(inc), str(d / "replay.cpp"), "-o",
+                    str(d / "replay.so")], check=True)
+    return ctypes.CDLL(str(d / "replay.so")).replay
+
+
+@pytest.mark.parametrize("W", [6, 7])
+@pytest.mark.parametrize("Nx,Ny,R", [(416, 416, 5), (100, 100, 24), (64, 70, 24), (128, 128, 9), (5, 7, 9), (9, 4, 7)])
+def test_spread_reads_only_taps_of_cells_on_the_grid(replay, Nx, Ny, R, W):
+    """The taps that the spread's threads apply, replayed on the host over the tables: exactly those of the cells on the
+    half grid, by modular arithmetic; none on a tile's rows or columns past it (grids whose sides are no multiple of the
+    tile's, and narrower than a tile). An offset outside 0 .. W-1 would read past the staged weights."""
+    ang = np.linspace(0, np.pi, R, endpoint=False) + 0.021
+    h = FourierHost(ang, Nx, Ny, max(Nx, Ny) + 3, float(max(Nx, Ny)), max(Nx, Ny) + 3.0, 0.2, np.pi / R, W=W)
+    tab = h.tables()
+    n = len(tab.tile_smp)
+    got = np.empty((n, 16, 16), np.int32)
+    arr = [np.ascontiguousarray(a, np.int32) for a in (tab.tile_ptr, tab.tile_smp, tab.kb)]
+    replay(*(a.ctypes.data_as(ctypes.c_void_p) for a in arr), tab.n_tiles, tab.n_tx, h.Mx, h.My, W,
+           got.ctypes.data_as(ctypes.c_void_p))
+    tile = np.repeat(np.arange(tab.n_tiles), np.diff(tab.tile_ptr))
+    mir = tab.tile_smp < 0
+    smp = np.where(mir, -tab.tile_smp - 1, tab.tile_smp)
+    sign = np.where(mir, -1, 1)[:, None]
+    q1 = (tile % tab.n_tx * 16)[:, None] + np.arange(16)
+    q2 = (tile // tab.n_tx * 16)[:, None] + np.arange(16)
+    d1 = ((sign * q1 - tab.kb[smp, :1]) % h.Mx)[:, None, :]
+    d2 = ((sign * q2 - tab.kb[smp, 1:]) % h.My)[:, :, None]
+    inside = (q1 <= h.Mx // 2)[:, None, :] & (q2 < h.My)[:, :, None]
+    want = np.where(inside & (d1 < W) & (d2 < W), d2 * W + d1, -1)
+    assert np.array_equal(got, want) and (want >= 0).any()
