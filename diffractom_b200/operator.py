@@ -845,7 +845,7 @@ class SinglePhaseForwardOperator:
                        self._s())
             return
         self._radon_fwd(src_ptr, z.data_ptr() + 2 * ib * self.Kstride, om, n, self.batches[ib]["K_batch"],
-                        sld=self.Ktot)
+                        sld=self.Ktot, m=m)
 
     def _pf_of(self, om, n):
         """(PF tensor, compact flag) for the tensor-core products over the n angles om: the stored PF of all angles,
