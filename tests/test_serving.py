@@ -47,3 +47,10 @@ def test_estimate_grows_with_the_request():
     assert estimate_request_bytes({**cfg, "Nx": 128, "Ny": 128}, 500, 3) > small
     assert estimate_request_bytes(cfg, 500, 8) > small
     assert estimate_request_bytes(cfg, 500, 3, precision="bf16") > small      # + the dense BF16 PF
+
+
+def test_a_request_s_reservation_covers_the_transpose_buffer():
+    """The operator's lines-fastest copies, which no other term of the estimate counts."""
+    from diffractom_b200.operator import SinglePhaseForwardOperator
+    from diffractom_b200.serving import WORKSPACE_BYTES
+    assert SinglePhaseForwardOperator.zt_max_bytes <= WORKSPACE_BYTES
