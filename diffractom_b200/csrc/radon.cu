@@ -516,7 +516,10 @@ __device__ __forceinline__ void ldrow(const __nv_bfloat16 *p, int o0, int, float
 // n_out-1], output row r for pixel plist[r] (the same arithmetic per pixel as the whole image). MODE as finish_run.
 // P channel groups of 256 per warp: the pixel's taps and weights are computed once for P x 8 channels per lane; every
 // channel sums the same terms in the same order whatever P is. Whole images with two taps per pixel and angle take
-// radon_backward_tile.
+// radon_backward_tile unless they have few pixels (launch_backward). Launches of few warps wait for one angle's chain
+// (place, loads, FMAs) after the other: the loop over the angles is unrolled, so that the next angles' places are
+// computed meanwhile (48 x 48 pixels, 180 angles, 256 channels 95 -> 62.5 us, BF16 rows 67 -> 58 us; unrolled by 4: 66
+// us), and the lane's first run is folded into the row pointer.
 template <int KERNEL, int MODE, typename ST, int P>
 __global__ void __launch_bounds__(32 * WARPS) radon_backward_v3(
     const ST *__restrict__ sino, int64_t sld, float *__restrict__ img, const float4 *__restrict__ geo, int n_angles, int nx,
@@ -546,8 +549,14 @@ __global__ void __launch_bounds__(32 * WARPS) radon_backward_v3(
 #pragma unroll
         for (int c = 0; c < CPL; ++c) acc[h][c] = 0.0f;
     const ST *col = sino + kblk;
+    if (P == 1) {
+        col += o[0][0];
+        o[0][1] -= o[0][0];
+        o[0][0] = 0;
+    }
     const int64_t angle_stride = (int64_t)ns * sld;
     if (data[0]) {
+#pragma unroll 8
         for (int a = 0; a < n_angles; ++a, col += angle_stride) {
             const AngleGeo g = unpack_geo(prm[a]);
             const float t = __fmaf_rn(g.A, g.rows_are_y ? fx : fy, __fmaf_rn(g.B, g.rows_are_y ? fy : fx, g.T0));
@@ -837,8 +846,14 @@ static int launch_backward(const ST *sino, int64_t sld, float *img, const float 
     const int64_t npix = plist ? n_list : (int64_t)nx * ny;
     const size_t smem = sizeof(AngleParams) * (size_t)(n_angles > 0 ? n_angles : 1);
     DFX_REQUIRE(smem <= 200 * 1024, "radon: %d angles exceed the shared memory of one launch", n_angles);
+    // Few warps (under 32 per SM with one pixel and 256 channels each): one warp per pixel and channel group, whose chain
+    // per angle is the shortest. Whole images, one pixel per warp against four, 90 angles: 48 x 48 pixels, 256 channels 33
+    // against 35 us, at 180 angles 62 and 97 (16 warps per SM); 64 x 64, 64 channels 44 and 52 (28); 80 x 80, 200 channels
+    // 75 and 55 (43); 128 x 128, 200 channels 138 and 112 (111). Over 16 x 16 to 256 x 256 pixels, 5 to 360 angles and 64
+    // to 1000 channels, float32 and BF16 rows, the line lies between 28 and 40 warps per SM.
+    const bool few = npix * cdiv(kstride, CPW) < 32 * 148;
     // pixels with at most two taps, an angle's rows within 32-bit byte offsets: neighbouring pixels share their bins
-    if (!plist && n_taps == 2 && (int64_t)n_det * sld * (int64_t)sizeof(ST) < ((int64_t)1 << 32)) {
+    if (!plist && !few && n_taps == 2 && (int64_t)n_det * sld * (int64_t)sizeof(ST) < ((int64_t)1 << 32)) {
         const dim3 tiles((unsigned)(cdiv(nx, TX) * cdiv(ny, BW)), (unsigned)cdiv(kstride, CPW));
         DFX_REQUIRE(cdiv(nx, TX) * cdiv(ny, BW) < 2147483647LL && tiles.y <= 65535u,
                     "radon: batch too large for one launch");
@@ -847,9 +862,9 @@ static int launch_backward(const ST *sino, int64_t sld, float *img, const float 
             lam, xb);
         return launch_status(MODE ? "radon_backward_spdhg" : "radon_backward");
     }
-    // two channel groups per warp once the batch has more than one (fewer, longer warps: the taps of a pixel are
-    // evaluated once for 16 channels per lane)
-    const bool pair = kstride > CPW;
+    // two channel groups per warp where the batch has them (the taps of a pixel are evaluated once for 16 channels per
+    // lane: 5 to 14 % faster from 40 warps per SM on), one where that leaves few warps (up to 1.7 times faster)
+    const bool pair = kstride > CPW && !few;
     dim3 grid((unsigned)cdiv(npix, WARPS), (unsigned)cdiv(kstride, pair ? 2 * CPW : CPW));
     DFX_REQUIRE(grid.x < 2147483647u && grid.y <= 65535u, "radon: batch too large for one launch");
     int st = pair ? allow_smem(radon_backward_v3<KERNEL, MODE, ST, 2>, smem)

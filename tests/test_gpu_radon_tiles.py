@@ -10,6 +10,10 @@ pytestmark = pytest.mark.gpu
 # (nx, ny, bins, angles, kb, kstride)
 SIZES = [(5, 4, 6, 3, 1, 8), (8, 7, 9, 9, 12, 16), (17, 21, 11, 13, 127, 128), (19, 16, 24, 8, 130, 136),
          (33, 30, 41, 17, 250, 256), (16, 18, 15, 16, 257, 264), (23, 9, 26, 7, 500, 504), (12, 35, 37, 5, 1000, 1008)]
+# the backprojection's four-pixel rows serve images of 4736 pixels x 256 channels on: sizes on both sides of that line
+# (one and two channel groups), widths around a row's four pixels, detectors narrower than the image
+LARGE = [(73, 65, 60, 3, 1, 8), (74, 64, 79, 9, 250, 256), (37, 128, 120, 8, 256, 256), (47, 50, 44, 17, 257, 264),
+         (49, 49, 55, 7, 500, 504), (131, 75, 90, 5, 127, 128)]
 
 
 def _geometry(nx, ny, bins, angles, kernel):
@@ -99,11 +103,12 @@ def test_bf16_image_table_forward_equals_the_float32_one():
 
 
 @pytest.mark.parametrize("kernel", ["trapezoid", "hat"])
-@pytest.mark.parametrize("size", SIZES, ids=str)
+@pytest.mark.parametrize("size", SIZES + LARGE, ids=str)
 def test_backprojection_of_whole_images_equals_the_pixel_lists(size, kernel):
-    """dfx_radon_backward (rows of pixels sharing bins) = dfx_radon_backward_pixels over every pixel (pixel by pixel),
-    bit for bit: float32 and BF16 rows with their own stride, padding channels 0; dfx_radon_backward_spdhg = the
-    backprojection followed by dfx_spdhg_primal_update, the padding channels of x, z kept."""
+    """dfx_radon_backward (rows of pixels sharing bins from 4736 warps on) = dfx_radon_backward_pixels over every pixel
+    (pixel by pixel, two channel groups per warp from as many warps on) and over a row of pixels, bit for bit: float32
+    and BF16 rows with their own stride, padding channels 0; dfx_radon_backward_spdhg = the backprojection followed by
+    dfx_spdhg_primal_update, the padding channels of x, z kept."""
     from diffractom_b200 import _lib
     nx, ny, bins, R, kb, ks = size
     rg = _geometry(nx, ny, bins, R, kernel)
@@ -122,6 +127,10 @@ def test_backprojection_of_whole_images_equals_the_pixel_lists(size, kernel):
     pixels(sino)
     _lib.call("dfx_radon_backward", sino.data_ptr(), out.data_ptr(), geo.data_ptr(), R, nx, ny, bins, ks, kb, kid, nt, s)
     assert torch.equal(out, want) and want.any() and not want[:, kb:].any()
+    row = torch.empty((nx, ks), device="cuda")         # a launch of few warps whatever the image
+    _lib.call("dfx_radon_backward_pixels", sino.data_ptr(), row.data_ptr(), geo.data_ptr(), R, nx, ny, bins, ks, kb, kid,
+              nt, pix[(ny // 2) * nx:].data_ptr(), nx, s)
+    assert torch.equal(row, want[(ny // 2) * nx:(ny // 2 + 1) * nx])
     # the primal step in the epilogue
     x, z, T = (torch.rand((nx * ny, ks), generator=g, device="cuda") for _ in range(3))
     x[:, kb:] = z[:, kb:] = T[:, kb:] = 0
