@@ -250,9 +250,9 @@ __device__ __forceinline__ void ldraw(const float *p, int o0, int o1, Raw8<float
     r.a = __ldg(reinterpret_cast<const float4 *>(p + o0));
     r.b = __ldg(reinterpret_cast<const float4 *>(p + o1));
 }
-__device__ __forceinline__ void ldraw(const __nv_bfloat16 *p, int o0, int, Raw8<__nv_bfloat16> &r)
+__device__ __forceinline__ void ldraw(const __nv_bfloat16 *p, Raw8<__nv_bfloat16> &r)
 {
-    r.u = __ldg(reinterpret_cast<const uint4 *>(p + o0));
+    r.u = __ldg(reinterpret_cast<const uint4 *>(p));
 }
 __device__ __forceinline__ void accraw(float (&a)[CPL], float w, const Raw8<float> &r) { acc8(a, w, r.a, r.b); }
 __device__ __forceinline__ void accraw(float (&a)[CPL], float w, const Raw8<__nv_bfloat16> &r)
@@ -264,22 +264,22 @@ __device__ __forceinline__ void accraw(float (&a)[CPL], float w, const Raw8<__nv
 // Table-driven forward: warp per (angle, bin, 256 channels), angle a of the launch = angles[a] of the table (angles
 // NULL: a); the same taps, weights and summation order as radon_forward_v4, so the same bits. Bound by the L1 data
 // path and L2 (a float32 launch of all 360 angles at 256 x 256 pixels, 1012 channels: 85 % and 80 % of their peaks);
-// what it needs is loads in flight at few registers: a software pipeline over groups of U taps, 2 of a float32 image
-// (60 registers; without it ptxas kept 40 and one tap's loads in flight) and 4 of a BF16 one. That launch went from 10.9
-// to 7.2 ms, 18 angles from 0.68 to 0.44 ms (U = 4: 8.1 and 0.46, U = 8: 11.7 and 0.64).
-template <typename ST, typename IT>
+// what it needs is loads in flight at few registers: a software pipeline over groups of U taps (60 registers; without
+// it ptxas kept 40 and one tap's loads in flight). That launch went from 10.9 to 7.2 ms, 18 angles from 0.68 to 0.44 ms
+// (U = 4: 8.1 and 0.46, U = 8: 11.7 and 0.64).
+template <typename ST>
 __global__ void __launch_bounds__(32 * WARPS) radon_forward_table(
-    const IT *__restrict__ img, ST *__restrict__ sino, int64_t sld, const int32_t *__restrict__ row_ptr,
+    const float *__restrict__ img, ST *__restrict__ sino, int64_t sld, const int32_t *__restrict__ row_ptr,
     const int2 *__restrict__ entries, const int32_t *__restrict__ angles, int ns, int kstride, int kb, float scale)
 {
-    constexpr int U = sizeof(IT) == 2 ? 4 : 2;
+    constexpr int U = 2;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int s = blockIdx.x * WARPS + warp;
     const int al = blockIdx.y;
     const int kblk = blockIdx.z * CPW;
     if (s >= ns) return;
     int k[2], o[2];
-    lane_runs<IT>(lane, kblk, kb, k, o);
+    lane_runs<float>(lane, kblk, kb, k, o);
     ST *out = sino + ((int64_t)al * ns + s) * sld;
     float acc[CPL];
 #pragma unroll
@@ -289,11 +289,11 @@ __global__ void __launch_bounds__(32 * WARPS) radon_forward_table(
         const int64_t r = (int64_t)a * ns + s;
         int e = __ldg(row_ptr + r);
         const int e1 = __ldg(row_ptr + r + 1);
-        const IT *base = img + kblk;
+        const float *base = img + kblk;
         // software pipeline over groups of U taps: the next group's pixels are loaded while this one's FMAs run
         if (e + U <= e1) {
             int2 t[U], tn[U];
-            Raw8<IT> q[U];
+            Raw8<float> q[U];
 #pragma unroll
             for (int i = 0; i < U; ++i) t[i] = __ldg(entries + e + i);
 #pragma unroll
@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(32 * WARPS) radon_forward_table(
             e += U;
 #pragma unroll 2
             for (; e + U <= e1; e += U) {
-                Raw8<IT> qn[U];
+                Raw8<float> qn[U];
 #pragma unroll
                 for (int i = 0; i < U; ++i) tn[i] = __ldg(entries + e + i);
 #pragma unroll
@@ -319,12 +319,70 @@ __global__ void __launch_bounds__(32 * WARPS) radon_forward_table(
         }
         for (; e < e1; ++e) {
             const int2 t = __ldg(entries + e);
-            Raw8<IT> q;
+            Raw8<float> q;
             ldraw(base + (int64_t)t.x * kstride, o[0], o[1], q);
             accraw(acc, __int_as_float(t.y), q);
         }
     }
     store_row(out, k, kstride, kb, scale, acc);
+}
+
+// The table-driven forward of a BF16 image with BF16 rows: the same split, 16 taps loaded before their FMAs. A warp's tap
+// is one 512-byte load, so that the wait for them counts, not L1: 0.281 ms for 18 angles at 256 x 256 pixels, 1012
+// channels, 17 us for 9 at 97 x 40, 256 channels; the pipeline above with groups of 4 taps 0.285 ms and 19 us, of 6 0.288
+// and 16, of 8 0.347 and 15.
+__global__ void __launch_bounds__(32 * WARPS) radon_forward_table_bf16(
+    const __nv_bfloat16 *__restrict__ img, __nv_bfloat16 *__restrict__ sino, int64_t sld,
+    const int32_t *__restrict__ row_ptr, const int2 *__restrict__ entries, const int32_t *__restrict__ angles, int ns,
+    int kstride, int kb, float scale)
+{
+    constexpr int U = 16;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int s = blockIdx.x * WARPS + warp;
+    const int al = blockIdx.y;
+    const int k = blockIdx.z * CPW + lane * CPL;
+    if (s >= ns) return;
+    const bool live = k < kstride;
+    __nv_bfloat16 *out = sino + ((int64_t)al * ns + s) * sld + k;
+    if (blockIdx.z * CPW >= kb) {
+        const float zero[CPL] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        if (live) st8(out, zero);
+        return;
+    }
+    const bool load = k < kb;
+    const int a = angles ? __ldg(angles + al) : al;
+    const int64_t r = (int64_t)a * ns + s;
+    int e = __ldg(row_ptr + r);
+    const int e1 = __ldg(row_ptr + r + 1);
+    const __nv_bfloat16 *base = img + (load ? k : 0);
+    float acc[CPL];
+#pragma unroll
+    for (int c = 0; c < CPL; ++c) acc[c] = 0.0f;
+    for (; e + U <= e1; e += U) {
+        int2 t[U];
+        Raw8<__nv_bfloat16> q[U];
+#pragma unroll
+        for (int i = 0; i < U; ++i) t[i] = __ldg(entries + e + i);
+#pragma unroll
+        for (int i = 0; i < U; ++i) {
+            q[i].u = make_uint4(0, 0, 0, 0);
+            if (load) ldraw(base + (int64_t)t[i].x * kstride, q[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < U; ++i) accraw(acc, __int_as_float(t[i].y), q[i]);
+    }
+    for (; e < e1; ++e) {
+        const int2 t = __ldg(entries + e);
+        Raw8<__nv_bfloat16> q;
+        q.u = make_uint4(0, 0, 0, 0);
+        if (load) ldraw(base + (int64_t)t.x * kstride, q);
+        accraw(acc, __int_as_float(t.y), q);
+    }
+    if (!live) return;
+    float o[CPL];
+#pragma unroll
+    for (int c = 0; c < CPL; ++c) o[c] = (k + c < kb) ? __fmul_rn(scale, acc[c]) : 0.0f;
+    st8(out, o);
 }
 
 // ------------------------------------------------------------------------------------------------ grouped table
@@ -922,8 +980,13 @@ static int radon_forward_table_any(const IT *img_k, ST *sino, int64_t sld, const
                 "multiple of %d >= kstride", (long long)sld, CPL);
     if (n_angles == 0) return DFX_OK;
     dim3 grid((unsigned)cdiv(n_det, WARPS), (unsigned)n_angles, (unsigned)cdiv(kstride, CPW));
-    radon_forward_table<ST, IT><<<grid, 32 * WARPS, 0, (cudaStream_t)stream>>>(
-        img_k, sino, sld, row_ptr, reinterpret_cast<const int2 *>(entries), angles, n_det, kstride, kb, scale);
+    const int2 *ent = reinterpret_cast<const int2 *>(entries);
+    if constexpr (sizeof(IT) == 2)
+        radon_forward_table_bf16<<<grid, 32 * WARPS, 0, (cudaStream_t)stream>>>(
+            img_k, sino, sld, row_ptr, ent, angles, n_det, kstride, kb, scale);
+    else
+        radon_forward_table<ST><<<grid, 32 * WARPS, 0, (cudaStream_t)stream>>>(
+            img_k, sino, sld, row_ptr, ent, angles, n_det, kstride, kb, scale);
     return launch_status("radon_forward_table");
 }
 
