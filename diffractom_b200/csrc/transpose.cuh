@@ -8,9 +8,9 @@ namespace dfx {
 // at in + m in_m (m = list[blockIdx.y], or m0 + blockIdx.y), out at out + blockIdx.y out_m. A lane transposes 4 x 4
 // elements in registers: four 16-byte loads along c, four 16-byte stores along r. The warp's 32 rows x 16 columns
 // read 64 contiguous bytes per row and write 128 per column; no shared memory, no synchronisation, and 64 bytes per
-// lane in flight. VI / VO: the vector form of the loads / stores (alignment); otherwise element by element.
-// HBM bounds it: 0.53 GB in and out 0.19 -> 0.09 ms against a 32 x 32 tile through shared memory with 4-byte loads.
-template <bool VI, bool VO>
+// lane in flight. VI: the loads may be vectors (alignment); otherwise element by element. The output's columns are
+// 16-byte aligned. HBM bounds it: 0.53 GB in and out 0.19 -> 0.09 ms against transpose_tile_kernel.
+template <bool VI>
 __global__ void __launch_bounds__(256) transpose_kernel(const float *__restrict__ in, int64_t in_ld, int64_t in_m,
                                                         const int32_t *__restrict__ list, int m0, float *__restrict__ out,
                                                         int64_t out_ld, int64_t out_m, int64_t rows, int64_t rows_out,
@@ -42,7 +42,7 @@ __global__ void __launch_bounds__(256) transpose_kernel(const float *__restrict_
     for (int j = 0; j < 4; ++j) {
         if (c + j >= cols) break;
         float *p = out + (c + j) * out_ld;
-        if (VO && r + 4 <= rows_out) {
+        if (r + 4 <= rows_out) {
             *reinterpret_cast<float4 *>(p) = make_float4(v[0][j], v[1][j], v[2][j], v[3][j]);
         } else {
 #pragma unroll
@@ -52,17 +52,47 @@ __global__ void __launch_bounds__(256) transpose_kernel(const float *__restrict_
     }
 }
 
+// The same for outputs whose columns are not 16-byte aligned (images of an odd number of pixels): a 32 x 32 tile through
+// shared memory, 128 contiguous bytes per warp on both sides. transpose_kernel's stores would be single words 16 bytes
+// apart: 9801 pixels, 1000 channels 29 us, so 21; 130 channels 10.6 and 6.5.
+static __global__ void __launch_bounds__(256) transpose_tile_kernel(
+    const float *__restrict__ in, int64_t in_ld, int64_t in_m, const int32_t *__restrict__ list, int m0,
+    float *__restrict__ out, int64_t out_ld, int64_t out_m, int64_t rows, int64_t rows_out, int64_t cols, int row_tiles)
+{
+    __shared__ float tile[32][33];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t r0 = (int64_t)(blockIdx.x % row_tiles) * 32, c0 = (int64_t)(blockIdx.x / row_tiles) * 32;
+    in += (list ? __ldg(list + blockIdx.y) : m0 + (int)blockIdx.y) * in_m;
+    out += blockIdx.y * out_m;
+    const bool cin = c0 + lane < cols, rout = r0 + lane < rows_out;
+    in += (r0 + warp) * in_ld + c0 + lane;
+    out += (c0 + warp) * out_ld + r0 + lane;
+    float v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = cin && r0 + warp + 8 * i < rows ? __ldg(in + 8 * i * in_ld) : 0.0f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) tile[warp + 8 * i][lane] = v[i];
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        if (rout && c0 + warp + 8 * i < cols) out[8 * i * out_ld] = tile[lane][warp + 8 * i];
+}
+
 inline int launch_transpose(const float *in, int64_t in_ld, int64_t in_m, const int32_t *list, int m0, float *out,
                             int64_t out_ld, int64_t out_m, int64_t rows, int64_t rows_out, int64_t cols, int n,
                             cudaStream_t st)
 {
-    const int64_t ct = cdiv(cols, 128), tiles = ct * cdiv(rows_out, 32);
-    DFX_REQUIRE(tiles < 2147483647LL && n <= 65535, "transpose: too large for one launch");
-    const bool vi = (uintptr_t)in % 16 == 0 && in_ld % 4 == 0 && in_m % 4 == 0;
     const bool vo = (uintptr_t)out % 16 == 0 && out_ld % 4 == 0 && out_m % 4 == 0;
-    const dim3 grid((unsigned)tiles, (unsigned)n);
-    const auto kernel = vi ? (vo ? transpose_kernel<true, true> : transpose_kernel<true, false>)
-                           : (vo ? transpose_kernel<false, true> : transpose_kernel<false, false>);
+    const int64_t rt = cdiv(rows_out, 32), ct = cdiv(cols, vo ? 128 : 32);
+    DFX_REQUIRE(rt * ct < 2147483647LL && n <= 65535, "transpose: too large for one launch");
+    const dim3 grid((unsigned)(rt * ct), (unsigned)n);
+    if (!vo) {
+        transpose_tile_kernel<<<grid, 256, 0, st>>>(in, in_ld, in_m, list, m0, out, out_ld, out_m, rows, rows_out, cols,
+                                                    (int)rt);
+        return launch_status("transpose");
+    }
+    const bool vi = (uintptr_t)in % 16 == 0 && in_ld % 4 == 0 && in_m % 4 == 0;
+    const auto kernel = vi ? transpose_kernel<true> : transpose_kernel<false>;
     kernel<<<grid, 256, 0, st>>>(in, in_ld, in_m, list, m0, out, out_ld, out_m, rows, rows_out, cols, (int)ct);
     return launch_status("transpose");
 }
