@@ -179,8 +179,9 @@ __global__ void __launch_bounds__(TC_THREADS) pf_tc_kernel(const __grid_constant
 }
 
 // BF16 copy of the data rows of the listed angles (blockIdx.y). PACKED: rows without padding (cp_pad = cp, a multiple of
-// 8) and 16-byte aligned arrays, so that an angle is one run of 8-element pieces; otherwise row by row. HBM bounds it: the
-// 360 angles of 263 x 2880 0.99 -> 0.24 ms against one element per thread with its row and column divided out.
+// 8) and 16-byte aligned arrays, so that an angle is one run of 8-element pieces; otherwise a block per row, or (up to
+// 128 columns) a warp per row. HBM bounds it: the 360 angles of 263 x 2880 0.99 -> 0.24 ms against one element per thread
+// with its row and column divided out; 360 angles of 40 x 13 padded to 16 6.6 us, 12.6 with a block per row.
 template <bool PACKED>
 __global__ void __launch_bounds__(256) rows_to_bf16_kernel(const float *__restrict__ in, __nv_bfloat16 *__restrict__ out,
                                                            const int32_t *__restrict__ omegas, int s0, int my, int cp,
@@ -199,8 +200,9 @@ __global__ void __launch_bounds__(256) rows_to_bf16_kernel(const float *__restri
             reinterpret_cast<uint4 *>(out)[i] = *reinterpret_cast<const uint4 *>(q);
         }
     } else {
-        for (int y = blockIdx.x; y < my; y += gridDim.x)
-            for (int j = threadIdx.x; j < cp_pad; j += 256)
+        const int tpr = cp_pad <= 128 ? 32 : 256, nr = 256 / tpr;          // threads per row, rows per block
+        for (int y = blockIdx.x * nr + threadIdx.x / tpr; y < my; y += gridDim.x * nr)
+            for (int j = threadIdx.x % tpr; j < cp_pad; j += tpr)
                 out[(int64_t)y * cp_pad + j] = __float2bfloat16_rn(j < cp ? __ldg(in + (int64_t)y * cp + j) : 0.0f);
     }
 }
@@ -376,7 +378,7 @@ extern "C" int dfx_rows_to_bf16(const float *in, void *out, const int32_t *omega
     DFX_REQUIRE(in && out, "rows_to_bf16: null pointer");
     DFX_REQUIRE(n_sub > 0 && my > 0 && cp > 0 && cp_pad >= cp, "rows_to_bf16: bad sizes");
     const bool packed = cp_pad == cp && cp % 8 == 0 && (uintptr_t)in % 16 == 0 && (uintptr_t)out % 16 == 0;
-    const int64_t per = packed ? cdiv((int64_t)my * cp / 8, 512) : my;
+    const int64_t per = packed ? cdiv((int64_t)my * cp / 8, 512) : cp_pad <= 128 ? cdiv(my, 8) : my;
     const auto kernel = packed ? rows_to_bf16_kernel<true> : rows_to_bf16_kernel<false>;
     for (int s0 = 0; s0 < n_sub; s0 += 65535) {
         const dim3 grid((unsigned)(per < 1024 ? per : 1024), (unsigned)(n_sub - s0 < 65535 ? n_sub - s0 : 65535));

@@ -66,7 +66,7 @@ def test_batch_support(npix, ks, kb, shift, mode, masked):
 
 
 @pytest.mark.parametrize("R,my,cp,pad,shift", [(3, 5, 16, 16, 0), (4, 7, 24, 24, 0), (2, 3, 13, 16, 0), (3, 1, 8, 8, 1),
-                                               (2, 263, 2880, 2880, 0)])
+                                               (2, 263, 2880, 2880, 0), (2, 19, 127, 128, 0), (2, 9, 129, 136, 0)])
 def test_rows_to_bf16(R, my, cp, pad, shift):
     from diffractom_b200 import _lib
     x = torch.empty(R * my * cp + 1, device="cuda")[shift:shift + R * my * cp].view(R, my, cp)
