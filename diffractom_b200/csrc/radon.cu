@@ -6,13 +6,16 @@
 // geometry only (detector coordinate, tap bins and weights) is the same for the whole warp: one warp instruction
 // serves 256 channels, and a zero weight skips its FMAs with a branch all lanes take.
 //
-// Forward (ray-driven gather, no atomics): a warp owns one bin of one angle; per image row it reads the two to four
-// pixels whose footprint reaches the bin. The grid is ordered so that one channel block of the image stays in L2
-// while all angles and bins of the launch read it.
+// Forward (ray-driven gather, no atomics): a warp owns one bin of one angle, or four neighbouring bins (grouped table);
+// it walks the pixels whose footprint reaches them, found per image row (radon_forward_v4) or listed in a table built
+// once per geometry. The grid is ordered so that one channel block of the image stays in L2 while all angles and bins
+// of the launch read it.
 //
-// Backward (pixel-driven, no atomics): a warp owns one pixel. The per-angle constants are computed once per block
-// into shared memory; per angle the warp evaluates the pixel's taps and reads 8 channels of each tap's sinogram bin
-// per lane. A fused variant applies SPDHG's primal step in the epilogue (no dz array).
+// Backward (pixel-driven, no atomics): a warp owns four neighbouring pixels of an image row (radon_backward_tile: whole
+// images, two taps per pixel and angle), or one pixel (radon_backward_v3: pixel lists, more taps, few pixels; the
+// per-angle constants are computed once per block into shared memory); per angle it evaluates the pixels' taps and
+// reads 8 channels of each tap's sinogram bin per lane. A fused variant applies SPDHG's primal step in the epilogue (no
+// dz array).
 //
 // The sinogram is float32 or, in the BF16 precision path, BF16 with its own row stride (bins of all orientation
 // batches side by side): loads widen BF16 to float32 exactly, the forward rounds its float32 sums once on store.
@@ -263,7 +266,7 @@ __device__ __forceinline__ void accraw(float (&a)[CPL], float w, const Raw8<__nv
 
 // Table-driven forward: warp per (angle, bin, 256 channels), angle a of the launch = angles[a] of the table (angles
 // NULL: a); the same taps, weights and summation order as radon_forward_v4, so the same bits. Bound by the L1 data
-// path and L2 (a float32 launch of all 360 angles at 256 x 256 pixels, 1012 channels: 85 % and 80 % of their peaks);
+// path and L2 (a float32 launch of all 360 angles at 256 x 256 pixels, 1012 channels: 84 % and 80 % of their peaks);
 // what it needs is loads in flight at few registers: a software pipeline over groups of U taps (60 registers; without
 // it ptxas kept 40 and one tap's loads in flight). That launch went from 10.9 to 7.2 ms, 18 angles from 0.68 to 0.44 ms
 // (U = 4: 8.1 and 0.46, U = 8: 11.7 and 0.64).
@@ -453,7 +456,7 @@ __global__ void ray_gtable_kernel(const float4 *__restrict__ geo, int n_angles, 
 // Grouped-table forward of a float32 image: warp per (angle, GB bins, 256 channels); U pixels in flight, each pixel's
 // FMAs into the bins whose weight is not 0 (a branch the whole warp takes). A block's warps take GA consecutive angles
 // of two groups: the rays of neighbouring angles through the same bins cross nearly the same pixels, so the block
-// finds them in L1 (hit rate 10 -> 70 %, L2 throughput 59 -> 23 % of its peak), which leaves the L1 data path as
+// finds them in L1 (hit rate 10 -> 64 %, L2 throughput 59 -> 28 % of its peak), which leaves the L1 data path as
 // its bound (76 %). 360 angles at 256 x 256 pixels, 1012 channels: 10.2 ms with a lane's 8 channels side by side, 7.6
 // with whole 512-byte loads (Chan), 6.6 with the block over angles (8 angles of one group: 6.7).
 constexpr int GA = 4;           // angles per block
@@ -666,10 +669,11 @@ __global__ void __launch_bounds__(32 * WARPS) radon_backward_v3(
 // takes is then a choice of registers, made by one switch per angle, which the whole warp takes alike, over the
 // 15 possible step patterns with straight-line code for each. The lanes compute the tap weights of BA angles in
 // parallel (lane = angle and pixel) and read them back as broadcasts. The terms and their order per pixel and channel
-// are radon_backward_v3's, so are the sums. BW rows below one another make a block: they share bins in L1 (67 % hits).
-// 256 x 256 pixels, 1012 channels, 360 angles: 8.7 -> 5.1 ms (BF16 rows 6.4 -> 4.2), 18 angles with SPDHG's primal
-// step 0.63 -> 0.41 ms. Latency is what is left (24 warps of 80 registers; L1 data path 60 %, issue 45 %): 6.2 ms at
-// 20 warps, 7.7 ms for 4 x 2 pixels with a switch per pixel, 5.5 ms for 512 channels per warp.
+// are radon_backward_v3's, so are the sums. BW rows below one another make a block: they share bins in L1 (65 % hits).
+// 256 x 256 pixels, 1012 channels, 360 angles: 8.2 ms with a pixel per warp, 5.0 so (with 8 neighbouring channels per
+// lane 10.8; BF16 rows 6.4 -> 4.1), 18 angles with SPDHG's primal step 0.49 -> 0.39 ms. Latency is what is left (24
+// warps of 80 registers; L1 data path 62 %, issue 52 %): 6.2 ms at 20 warps, 7.7 ms for 4 x 2 pixels with a switch per
+// pixel, 5.5 ms for 512 channels per warp.
 constexpr int TX = 4;                           // pixels of a warp
 constexpr int BW = 4;                           // warps per block: rows below one another
 constexpr int BA = 32 / TX;                     // angles per weight batch (one lane per angle and pixel)
@@ -903,13 +907,16 @@ static int launch_backward(const ST *sino, int64_t sld, float *img, const float 
 {
     const int64_t npix = plist ? n_list : (int64_t)nx * ny;
     const size_t smem = sizeof(AngleParams) * (size_t)(n_angles > 0 ? n_angles : 1);
+    // radon_backward_v3's limit, for both kernels alike: which one serves a launch depends on its size
     DFX_REQUIRE(smem <= 200 * 1024, "radon: %d angles exceed the shared memory of one launch", n_angles);
-    // Few warps (under 32 per SM with one pixel and 256 channels each): one warp per pixel and channel group, whose chain
-    // per angle is the shortest. Whole images, one pixel per warp against four, 90 angles: 48 x 48 pixels, 256 channels 33
-    // against 35 us, at 180 angles 62 and 97 (16 warps per SM); 64 x 64, 64 channels 44 and 52 (28); 80 x 80, 200 channels
-    // 75 and 55 (43); 128 x 128, 200 channels 138 and 112 (111). Over 16 x 16 to 256 x 256 pixels, 5 to 360 angles and 64
-    // to 1000 channels, float32 and BF16 rows, the line lies between 28 and 40 warps per SM.
-    const bool few = npix * cdiv(kstride, CPW) < 32 * 148;
+    // Few warps (under 28 per SM with one pixel and 256 channels each, 32 with the primal step, 24 for BF16 rows): one
+    // warp per pixel and channel group, whose chain per angle is the shortest. Whole images, one pixel per warp against
+    // four, 90 angles, without the primal step, with it, and BF16 rows: 48 x 48 pixels, 256 channels (16 per SM) 34 and
+    // 50 us, 34 and 52, 32 and 44; 64 x 64, 64 channels (28) 44 and 52, 46 and 52, 46 and 48; 48 x 48, 400 channels (31)
+    // 46 and 53, 46 and 55, 48 and 48, but at 12 angles 35.3 and 34.3 for a call without the step; 64 x 40, 400 channels
+    // (35) 56 and 54, 60 and 56, 59 and 50; 80 x 80, 200 channels (43) 75 and 55, 77 and 58, 67 and 50.
+    constexpr int line = sizeof(ST) == 2 ? 24 : MODE == 1 ? 32 : 28;
+    const bool few = npix * cdiv(kstride, CPW) < line * 148;
     // pixels with at most two taps, an angle's rows within 32-bit byte offsets: neighbouring pixels share their bins
     if (!plist && !few && n_taps == 2 && (int64_t)n_det * sld * (int64_t)sizeof(ST) < ((int64_t)1 << 32)) {
         const dim3 tiles((unsigned)(cdiv(nx, TX) * cdiv(ny, BW)), (unsigned)cdiv(kstride, CPW));

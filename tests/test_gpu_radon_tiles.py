@@ -10,10 +10,12 @@ pytestmark = pytest.mark.gpu
 # (nx, ny, bins, angles, kb, kstride)
 SIZES = [(5, 4, 6, 3, 1, 8), (8, 7, 9, 9, 12, 16), (17, 21, 11, 13, 127, 128), (19, 16, 24, 8, 130, 136),
          (33, 30, 41, 17, 250, 256), (16, 18, 15, 16, 257, 264), (23, 9, 26, 7, 500, 504), (12, 35, 37, 5, 1000, 1008)]
-# the backprojection's four-pixel rows serve images of 4736 pixels x 256 channels on: sizes on both sides of that line
-# (one and two channel groups), widths around a row's four pixels, detectors narrower than the image
+# the backprojection's four-pixel rows serve images of 3552 (BF16 rows), 4144 or 4736 (with the primal step) pixels x 256
+# channels on: sizes on both sides of those lines (one and two channel groups), widths around a row's four pixels,
+# detectors narrower than the image
 LARGE = [(73, 65, 60, 3, 1, 8), (74, 64, 79, 9, 250, 256), (37, 128, 120, 8, 256, 256), (47, 50, 44, 17, 257, 264),
-         (49, 49, 55, 7, 500, 504), (131, 75, 90, 5, 127, 128)]
+         (49, 49, 55, 7, 500, 504), (131, 75, 90, 5, 127, 128), (56, 74, 70, 6, 129, 136), (53, 67, 60, 11, 30, 32),
+         (41, 51, 48, 10, 300, 304)]
 
 
 def _geometry(nx, ny, bins, angles, kernel):
@@ -105,10 +107,10 @@ def test_bf16_image_table_forward_equals_the_float32_one():
 @pytest.mark.parametrize("kernel", ["trapezoid", "hat"])
 @pytest.mark.parametrize("size", SIZES + LARGE, ids=str)
 def test_backprojection_of_whole_images_equals_the_pixel_lists(size, kernel):
-    """dfx_radon_backward (rows of pixels sharing bins from 4736 warps on) = dfx_radon_backward_pixels over every pixel
-    (pixel by pixel, two channel groups per warp from as many warps on) and over a row of pixels, bit for bit: float32
-    and BF16 rows with their own stride, padding channels 0; dfx_radon_backward_spdhg = the backprojection followed by
-    dfx_spdhg_primal_update, the padding channels of x, z kept."""
+    """dfx_radon_backward (rows of pixels sharing bins from a few thousand warps on) = dfx_radon_backward_pixels over
+    every pixel (pixel by pixel, two channel groups per warp from as many warps on) and over a row of pixels, bit for
+    bit: float32 and BF16 rows with their own stride, padding channels 0; dfx_radon_backward_spdhg = the backprojection
+    followed by dfx_spdhg_primal_update, the padding channels of x, z kept."""
     from diffractom_b200 import _lib
     nx, ny, bins, R, kb, ks = size
     rg = _geometry(nx, ny, bins, R, kernel)
