@@ -202,8 +202,9 @@ __global__ void __launch_bounds__(FR_TS *FR_TS) fr_spread_kernel(
         }
         __syncthreads();
         // a warp holds two rows of the tile: of 32 samples at a time, those with a tap on one of the rows (a ballot
-        // instead of a try per thread, and two channels per shared load: 1.30 -> 1.08 ms per slice of 128 channels at 416 x
-        // 416 pixels and 360 angles; broadcasts of the staged values bound it)
+        // instead of a try per thread, and two channels per shared load: 1.30 -> 1.11 ms per slice of 128 channels at
+        // 416 x 416 pixels and 360 angles; what is left is the wait for the block's slowest warp at the end of a round,
+        // the largest stall, beside issue at 57 % and the L1 data path at 44 %)
         const int row0 = fr_cell((tile / n_tx) * FR_TS + (ly & ~1), My);
         for (int h = 0; h < nb; h += 32) {
             const int u = h + (lid & 31);

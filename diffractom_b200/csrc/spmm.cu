@@ -10,9 +10,9 @@
 // per thread, the whole data row staged at once); the forward over stored copies runs over eta blocks
 // (spmm_forward_b4_kernel), the CSR kernel serving generated copies. The lines-fastest forms turn the work around:
 // the dense operand (the Radon output for the forward, the data rows for the adjoint) is first transposed to detector
-// lines fastest, then a warp walks one row's entries with its lanes on the lines, reading every entry once and a
-// whole 128-byte segment of the column per 32 lines (spmm_forward_zt_kernel, spmm_adjoint_zt_kernel); their sums
-// are the kernels' above bit for bit.
+// lines fastest, then a warp walks one row's entries with its lanes on the lines, reading every entry once and the
+// column's lines in contiguous segments, 512 bytes per load of 128 lines (ZtLines; spmm_forward_zt_kernel,
+// spmm_adjoint_zt_kernel); their sums are the kernels' above bit for bit.
 #include "dfx_common.cuh"
 #include "transpose.cuh"
 
@@ -420,8 +420,9 @@ __global__ void __launch_bounds__(SP_ROWS) spmm_forward_b4_kernel(
 // of Z column k in 512-byte segments, several entries in flight, and applies the entry's four values with paired fused
 // multiply-adds (fma.rn.f32x2: two IEEE fmaf in one instruction, lines t and t + 1). Instructions bounded it: with a
 // 4-byte load per 32 lines, each guarded, 92 per entry, now 65 (2.27 -> 1.86 ms for the 360 angles of 256 x 256 pixels,
-// 1012 channels, transposes in; 0.64 -> 0.56 for the 180 of 99 x 99); what is left is L2 latency at 24 warps. A block of 8 warps owns the block rows of nb consecutive eta blocks, all rings (nb * P <= 16 rows; one eta
-// block above 16 rings), whose outputs j = 4 cb P .. 4 (cb + nb) P - 1 are contiguous in a data row. The rows differ
+// 1012 channels, transposes in; 0.64 -> 0.56 for the 180 of 99 x 99); what is left is L2 latency at 24 warps. A block
+// of 8 warps owns the block rows of nb consecutive eta blocks, all rings (nb * P <= 16 rows; one eta block above 16
+// rings), whose outputs j = 4 cb P .. 4 (cb + nb) P - 1 are contiguous in a data row. The rows differ
 // in length, so the warps take them longest first from a shared counter instead of one row each: the block no longer
 // waits for its longest row with most warps idle. The sums go to shared memory; the block's data row segments, put in
 // L2 by a prefetch when the block starts, are then read a batch of lines at a time and written back whole. The sums
@@ -641,12 +642,12 @@ __global__ void __launch_bounds__(256, WIDE ? 3 : 2) spmm_forward_zt_kernel(
 // dt[s][j][y] (line stride ly, lines my .. ly - 1 zero): the data rows of one launch's angles with the detector lines
 // fastest. A warp owns kw (1, 2 or 4) consecutive orientation rows k of one angle, one after the other, and up to
 // 32 ZT_G lines (ZtLines); per entry (j, v) of a row it reads the entry once and column j's lines in 512-byte
-// segments, several entries in flight, paired fused multiply-adds. L2 bounds it (76 % of its peak at 288 lines: every
+// segments, several entries in flight, paired fused multiply-adds. L2 bounds it (82 % of its peak at 288 lines: every
 // entry reads a column from there). With a guarded 4-byte load per 32 lines, 43 instructions per entry, the 360
-// angles of 256 x 256 pixels, 1012 channels took 3.94 ms (transposes in), now 3.38; 180 of 99 x 99 0.83, now 0.59. A block's 8 warps
-// hold 8 kw consecutive orientations, written as whole row segments of the Radon input through shared memory (kw is
-// the largest that still gives the launch a few waves of blocks). Per output the sum runs over the row's entries in
-// order with fmaf from 0 and is scaled by alpha: spmm_adjoint8_kernel's bits.
+// angles of 256 x 256 pixels, 1012 channels took 3.94 ms (transposes in), now 3.38; 180 of 99 x 99 0.83, now 0.59. A
+// block's 8 warps hold 8 kw consecutive orientations, written as whole row segments of the Radon input through shared
+// memory (kw is the largest that still gives the launch a few waves of blocks). Per output the sum runs over the row's
+// entries in order with fmaf from 0 and is scaled by alpha: spmm_adjoint8_kernel's bits.
 constexpr int AZ_KW = 4;                 // orientation rows per warp at most
 constexpr int AZ_WARPS = 8;
 
@@ -840,16 +841,23 @@ static int launch_zt(const float *zt, const int32_t *fb_ptr, const uint16_t *fb_
 {
     int dev = 0, nsm = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    // fewer blocks than SMs: fewer eta blocks each (12 angles of 90 eta bins x 3 rings, 53 lines: 60 blocks of 15 rows
-    // 44 us, 276 of 3 rows 28 us; at 18 angles of 180 x 5, 103 lines, 270 blocks of 15 rows are the faster ones, 69
-    // against 87 us with 5 rows: the rows are taken longest first and the write-back has whole segments)
+    // fewer blocks than SMs: fewer eta blocks each. 48 x 48 pixels, 90 eta bins x 3 rings, 53 lines: 12 angles, 60 blocks
+    // of 15 rows, 38 -> 31 us; 5 angles 39 -> 29; 64 x 64, 120 x 5, 70 lines, 60 blocks 49 -> 43; 128 x 128, 120 x 5,
+    // 133 lines, 90 blocks 62 -> 56; 99 x 99, 180 x 5, 103 lines, 135 blocks 52 -> 55. Not further: with two blocks per
+    // SM as the line 270 blocks of 99 x 99 64 -> 90 us, 180 of 128 x 128 78 -> 90, 162 of 80 x 80 31 -> 25: the rows are
+    // taken longest first and the write-back has whole segments.
     while (nb > 1 && cdiv(ncb, nb) * nyb * na < nsm) --nb;
-    // from four waves on three blocks of 80 registers per SM with three entries in flight per warp are the faster ones
-    // (360 angles at 256 x 256 pixels, 1012 channels, both transposes in: 1.86 against 2.05 ms; 180 at 99 x 99: 0.56
-    // against 0.63), below two of 128 with four entries (18 angles at 99 x 99: 69 against 74 us)
-    if (MT > 2 && cdiv(ncb, nb) * nyb * na >= 4LL * 3 * nsm)
-        return launch_zt_as<MT, true>(zt, fb_ptr, fb_k, fb_v, fb_mask, data, omegas, r0, na, my, ly, nyb, P, C, ncb, nb,
-                                      kb, st);
+    // three blocks of 80 registers per SM with three entries in flight per warp, or two of 128 with four. From four
+    // waves of three on the former: 36 waves (360 angles at 256 x 256 pixels, 1012 channels) 1.67 against 1.87 ms, 6
+    // waves (180 at 99 x 99) 0.53 against 0.60, 4.1 waves 0.187 against 0.199. Under a wave the latter: 0.6 waves (18
+    // angles at 99 x 99) 64 against 76 us, 1.0 (45 at 128 x 128) 157 against 181. Between them the former is 5 to 19 %
+    // ahead from 1.5 waves on (36 angles at 256 x 256, 3.6 waves: 203 against 220 us; 120 at 64 x 64, 2.7: 204 against
+    // 253): there the rule is not yet at its best.
+    if constexpr (MT > 2) {
+        if (cdiv(ncb, nb) * nyb * na >= 4LL * 3 * nsm)
+            return launch_zt_as<MT, true>(zt, fb_ptr, fb_k, fb_v, fb_mask, data, omegas, r0, na, my, ly, nyb, P, C, ncb,
+                                          nb, kb, st);
+    }
     return launch_zt_as<MT, false>(zt, fb_ptr, fb_k, fb_v, fb_mask, data, omegas, r0, na, my, ly, nyb, P, C, ncb, nb, kb,
                                    st);
 }

@@ -36,7 +36,7 @@ AUTO_FFT_PIXELS = 400 * 400   # projector="auto": the Fourier-slice projector fo
 SPARSE_MIN_BATCHES = 4    # sparse modes: at least this many batches (SPFO:135)
 CAND_BYTES = 2 + 4 + 4 + 4 + 4          # per candidate / non-zero scratch of the reference's generator
 NNZ_BYTES = 2 + 4 + 4 + 2 + 4 + 2 + 4   # (pf_generate.py:29-30), used by the batch-size rule
-GTABLE_MIN_WARPS = 3 * 148 * 32          # forwards of a scan with this many grouped-table warps read the grouped table
+GTABLE_MIN_WARPS = 3 * 148 * 32          # whole scans of three waves of grouped-table warps on read the grouped table
 KSTRIDE_ALIGN = 16                       # channel stride of the batch buffers (16 channels per tensor-memory load)
 
 
@@ -57,11 +57,11 @@ class SinglePhaseForwardOperator:
     # neighbouring eta bins of a ring per entry; the same sums bit for bit); False: over the forward CSR itself
     forward_blocks = True
     # the blocked forward products read the Radon output transposed to detector lines fastest (one warp per block
-    # row, whole 128-byte segments of a Z column per entry; dfx_spmm_pf_forward_blocked_zt, the same bits) through a
+    # row, whole line segments of a Z column per entry; dfx_spmm_pf_forward_blocked_zt, the same bits) through a
     # buffer of up to zt_max_angles angles of a batch; False: dfx_spmm_pf_forward_blocked on the channel-fastest output
     forward_lines_fastest = True
     # the adjoint products read the data rows transposed to detector lines fastest (one warp per orientation row,
-    # whole 128-byte segments of a data column per entry; dfx_spmm_pf_adjoint_zt, the same bits) through the same
+    # whole line segments of a data column per entry; dfx_spmm_pf_adjoint_zt, the same bits) through the same
     # buffer; False: dfx_spmm_pf_adjoint on the segment-fastest rows
     adjoint_lines_fastest = True
     # the transpose buffer: a chunk's angles and its bytes at most (at least one angle). Fewer angles leave launches
@@ -384,11 +384,14 @@ class SinglePhaseForwardOperator:
         om_ptr = None if om is None else om.data_ptr()
         rp, ent = (self._ray_rp, self._ray_ent) if ray is None else ray[:2]
         grp = self._ray_grp if ray is None else (ray[3] if len(ray) > 3 else None)
-        # a scan's consecutive angles share their pixels in L1 through the grouped table, a subset's do not (18 angles
-        # at 256 x 256 pixels, 1012 channels: 0.75 ms grouped, 0.44 ms per-bin; all 360: 6.6 and 7.2 ms). It has a
-        # quarter of the warps: below about three waves of them the per-bin table is the faster one (180 angles of 99
-        # x 99 pixels, 4 waves: 0.53 grouped, 0.56 ms per-bin; 91 of 131 x 131 pixels, 333 channels, 1.3 waves: 0.31
-        # and 0.26 ms; 90 of 48 x 48, half a wave: 0.069 and 0.048 ms)
+        # a scan's consecutive angles share their pixels in L1 through the grouped table; it has a quarter of the warps.
+        # Whole scans, grouped and per-bin, by waves of grouped warps (148 x 32): 0.5 waves (48 x 48 pixels, 90 angles)
+        # 68 and 48 us, 2.5 (160 x 160, 140) 614 and 570, 2.5 (80 x 80, 180) 283 and 269, 3.1 (64 x 64, 270) 254 and
+        # 261, 3.1 (131 x 131, 140) 591 and 572, 3.3 (99 x 99, 150) 456 and 472, 3.3 (256 x 256, 120) 1319 and 1259, 4.0
+        # (99 x 99, 180) 534 and 561, 5.0 (256 x 256, 180) 1808 and 1866, 20 (360) 6666 and 7318: equal within 5 % about
+        # three waves. The angles of interleaved subsets lie further apart and share less; 360 angles at 256 x 256,
+        # 1012 channels: every 20th 749 and 417 us, 8th 1187 and 958, 4th 1911 and 1861, 3rd 2445 and 2483, 2nd 3481 and
+        # 3695: subsets read the per-bin table (a scan in two subsets would gain 4 to 7 % from the grouped one)
         warps = n_ang * -(-self.My // 4) * -(-self.Kstride // 256)
         if grp is not None and m is None and warps >= GTABLE_MIN_WARPS:
             out = (dst_ptr,) if sld is None else (dst_ptr, sld)
