@@ -414,20 +414,21 @@ __global__ void __launch_bounds__(SP_ROWS) spmm_forward_b4_kernel(
 }
 
 // ---- blocked forward over the lines-fastest sinogram ----
-// zt[s][k][y] (line stride ly = 32 * groups, lines my .. ly - 1 zero) is the Radon output of one launch's angles with
-// the detector lines fastest. A warp applies one block row (four eta bins of one ring) of one angle at a time to up
-// to 32 ZT_G lines (ZtLines). Per entry the warp reads the entry once (the same address in every lane) and the lines
-// of Z column k in 512-byte segments, several entries in flight, and applies the entry's four values with paired fused
-// multiply-adds (fma.rn.f32x2: two IEEE fmaf in one instruction, lines t and t + 1). Instructions bounded it: with a
-// 4-byte load per 32 lines, each guarded, 92 per entry, now 65 (2.27 -> 1.86 ms for the 360 angles of 256 x 256 pixels,
-// 1012 channels, transposes in; 0.64 -> 0.56 for the 180 of 99 x 99); what is left is L2 latency at 24 warps. A block
-// of 8 warps owns the block rows of nb consecutive eta blocks, all rings (nb * P <= 16 rows; one eta block above 16
-// rings), whose outputs j = 4 cb P .. 4 (cb + nb) P - 1 are contiguous in a data row. The rows differ
-// in length, so the warps take them longest first from a shared counter instead of one row each: the block no longer
-// waits for its longest row with most warps idle. The sums go to shared memory; the block's data row segments, put in
-// L2 by a prefetch when the block starts, are then read a batch of lines at a time and written back whole. The sums
-// per output run over the block row's entries in order with fmaf, each added once to the data row, as in
-// spmm_forward_b4_kernel: the results are that kernel's (and the CSR kernel's) bit for bit.
+// zt[s][k][y] (line stride ly = 32 * groups, lines my .. ly - 1 zero) is the Radon output of one launch's angles
+// with the detector lines fastest. A warp applies one block row (four eta bins of one ring) of one angle at a time
+// to up to 32 ZT_G lines (ZtLines). Per entry the warp reads the entry once (the same address in every lane) and the
+// lines of Z column k in 512-byte segments, several entries in flight, and applies the entry's four values with
+// paired fused multiply-adds (fma.rn.f32x2: two IEEE fmaf in one instruction, lines t and t + 1). Instructions
+// bounded it with a 4-byte load per 32 lines, each guarded: 2.27 -> 1.70 ms for the 360 angles of 256 x 256 pixels,
+// 1012 channels, transposes in, 0.64 -> 0.53 for the 180 of 99 x 99; now 73 instructions per entry, issue at 57 %,
+// and what is left is L2 latency at 24 warps. A block of 8 warps owns the block rows of nb consecutive eta blocks,
+// all rings (nb * P <= 16 rows; one eta block above 16 rings), whose outputs j = 4 cb P .. 4 (cb + nb) P - 1 are
+// contiguous in a data row. The rows differ in length, so the warps take them longest first from a shared counter
+// instead of one row each: the block no longer waits for its longest row with most warps idle. The sums go to shared
+// memory; the block's data row segments, put in L2 by a prefetch when the block starts, are then read a batch of
+// lines at a time and written back whole. The sums per output run over the block row's entries in order with fmaf,
+// each added once to the data row, as in spmm_forward_b4_kernel: the results are that kernel's (and the CSR
+// kernel's) bit for bit.
 constexpr int ZT_G = 9;                  // 32-line groups per warp at most (288 lines)
 // entries in flight per warp for MT line groups
 constexpr int zt_uf(int mt, bool wide) { return mt <= 2 ? 8 : wide ? 3 : 4; }
@@ -639,15 +640,15 @@ __global__ void __launch_bounds__(256, WIDE ? 3 : 2) spmm_forward_zt_kernel(
 }
 
 // ---- adjoint over the lines-fastest data rows ----
-// dt[s][j][y] (line stride ly, lines my .. ly - 1 zero): the data rows of one launch's angles with the detector lines
-// fastest. A warp owns kw (1, 2 or 4) consecutive orientation rows k of one angle, one after the other, and up to
-// 32 ZT_G lines (ZtLines); per entry (j, v) of a row it reads the entry once and column j's lines in 512-byte
-// segments, several entries in flight, paired fused multiply-adds. L2 bounds it (82 % of its peak at 288 lines: every
-// entry reads a column from there). With a guarded 4-byte load per 32 lines, 43 instructions per entry, the 360
-// angles of 256 x 256 pixels, 1012 channels took 3.94 ms (transposes in), now 3.38; 180 of 99 x 99 0.83, now 0.59. A
-// block's 8 warps hold 8 kw consecutive orientations, written as whole row segments of the Radon input through shared
-// memory (kw is the largest that still gives the launch a few waves of blocks). Per output the sum runs over the row's
-// entries in order with fmaf from 0 and is scaled by alpha: spmm_adjoint8_kernel's bits.
+// dt[s][j][y] (line stride ly, lines my .. ly - 1 zero): the data rows of one launch's angles with the detector
+// lines fastest. A warp owns kw (1, 2 or 4) consecutive orientation rows k of one angle, one after the other, and up
+// to 32 ZT_G lines (ZtLines); per entry (j, v) of a row it reads the entry once and column j's lines in 512-byte
+// segments, several entries in flight, paired fused multiply-adds. L2 bounds it (82 % of its peak at 288 lines:
+// every entry reads a column from there; 24 instructions per entry). With a guarded 4-byte load per 32 lines the 360
+// angles of 256 x 256 pixels, 1012 channels took 3.94 ms (transposes in), now 2.9; 180 of 99 x 99 0.83, now 0.53. A
+// block's 8 warps hold 8 kw consecutive orientations, written as whole row segments of the Radon input through
+// shared memory (kw is the largest that still gives the launch a few waves of blocks). Per output the sum runs over
+// the row's entries in order with fmaf from 0 and is scaled by alpha: spmm_adjoint8_kernel's bits.
 constexpr int AZ_KW = 4;                 // orientation rows per warp at most
 constexpr int AZ_WARPS = 8;
 
