@@ -580,8 +580,10 @@ __device__ __forceinline__ void ldrow(const __nv_bfloat16 *p, int o0, int, float
 // radon_backward_tile unless they have few pixels (launch_backward). Launches of few warps wait for one angle's chain
 // (place, loads, FMAs) after the other: the loop over the angles is unrolled, so that the next angles' places are
 // computed meanwhile (48 x 48 pixels, 180 angles, 256 channels 95 -> 62.5 us, BF16 rows 67 -> 58 us; unrolled by 4: 66
-// us), and the lane's first run is folded into the row pointer.
-template <int KERNEL, int MODE, typename ST, int P>
+// us), and the lane's first run is folded into the row pointer. PAIRS (P = 1, more than two taps): two taps' rows loaded
+// before their FMAs, 164 -> 114 us in that launch with four taps; with P = 2 it costs registers (1.02 -> 1.27 ms for 99 x
+// 99 pixels, 1000 channels), with two taps code (62.5 -> 65 us).
+template <int KERNEL, int MODE, typename ST, int P, bool PAIRS>
 __global__ void __launch_bounds__(32 * WARPS) radon_backward_v3(
     const ST *__restrict__ sino, int64_t sld, float *__restrict__ img, const float4 *__restrict__ geo, int n_angles, int nx,
     int ny, int ns, int kstride, int kb, int n_taps, float *__restrict__ z, const float *__restrict__ T, float inv_p,
@@ -634,6 +636,25 @@ __global__ void __launch_bounds__(32 * WARPS) radon_backward_v3(
                     ldrow(col + h * CPW + (int64_t)(sf + 1) * sld, o[h][0], o[h][1], b0, b1);
                     acc8(acc[h], w0, a0, a1);
                     acc8(acc[h], w1, b0, b1);
+                }
+                continue;
+            }
+            if constexpr (PAIRS) {
+                for (int i = 0; i < ntap; i += 2) {
+                    float ww[2];
+                    bool on[2];
+                    float4 q[2][2];
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        const int s = sf + i + j;
+                        const float w = tap_weight<KERNEL>(g, __fsub_rn(t, (float)s));
+                        on[j] = i + j < ntap && s >= 0 && s < ns && w != 0.0f;
+                        ww[j] = __fmul_rn(g.w, w);
+                        if (on[j]) ldrow(col + (int64_t)s * sld, o[0][0], o[0][1], q[j][0], q[j][1]);
+                    }
+#pragma unroll
+                    for (int j = 0; j < 2; ++j)
+                        if (on[j]) acc8(acc[0], ww[j], q[j][0], q[j][1]);
                 }
                 continue;
             }
@@ -932,17 +953,14 @@ static int launch_backward(const ST *sino, int64_t sld, float *img, const float 
     const bool pair = kstride > CPW && !few;
     dim3 grid((unsigned)cdiv(npix, WARPS), (unsigned)cdiv(kstride, pair ? 2 * CPW : CPW));
     DFX_REQUIRE(grid.x < 2147483647u && grid.y <= 65535u, "radon: batch too large for one launch");
-    int st = pair ? allow_smem(radon_backward_v3<KERNEL, MODE, ST, 2>, smem)
-                  : allow_smem(radon_backward_v3<KERNEL, MODE, ST, 1>, smem);
+    const auto kernel = pair ? radon_backward_v3<KERNEL, MODE, ST, 2, false>
+                        : KERNEL == 1 && n_taps > 2 ? radon_backward_v3<KERNEL, MODE, ST, 1, KERNEL == 1>
+                                                    : radon_backward_v3<KERNEL, MODE, ST, 1, false>;
+    const int st = allow_smem(kernel, smem);
     if (st) return st;
-    if (pair)
-        radon_backward_v3<KERNEL, MODE, ST, 2><<<grid, 32 * WARPS, smem, (cudaStream_t)stream>>>(
-            sino, sld, img, reinterpret_cast<const float4 *>(geo), n_angles, nx, ny, n_det, kstride, kb, n_taps, z, T,
-            inv_p, lam, xb, plist, npix);
-    else
-        radon_backward_v3<KERNEL, MODE, ST, 1><<<grid, 32 * WARPS, smem, (cudaStream_t)stream>>>(
-            sino, sld, img, reinterpret_cast<const float4 *>(geo), n_angles, nx, ny, n_det, kstride, kb, n_taps, z, T,
-            inv_p, lam, xb, plist, npix);
+    kernel<<<grid, 32 * WARPS, smem, (cudaStream_t)stream>>>(sino, sld, img, reinterpret_cast<const float4 *>(geo),
+                                                             n_angles, nx, ny, n_det, kstride, kb, n_taps, z, T, inv_p,
+                                                             lam, xb, plist, npix);
     return launch_status(MODE ? "radon_backward_spdhg" : "radon_backward");
 }
 

@@ -173,3 +173,46 @@ def test_backprojection_with_more_than_two_taps():
     want = torch.einsum("abp,abk->pk", A[:, :, :nx * ny].double(), sino.double())
     bound = torch.einsum("abp,abk->pk", A[:, :, :nx * ny].double().abs(), sino.double().abs()) * 2 * R * 4 * 2.0 ** -24
     assert ((out.double() - want).abs()[:, :kb] <= bound[:, :kb]).all() and not out[:, kb:].any()
+
+
+@pytest.mark.parametrize("bins,width,taps", [(150, 140.0, 3), (301, 280.0, 5), (90, 140.0, 3)])
+@pytest.mark.parametrize("ks,kb", [(304, 300), (8, 5)])
+def test_more_than_two_taps_two_at_a_time(bins, width, taps, ks, kb):
+    """Three to five taps a pixel, detectors wider and narrower than the image: a row of pixels (few warps, the taps'
+    rows loaded in pairs) = the same pixels of the whole image (two channel groups per warp at 304 channels) bit for
+    bit, float32 and BF16 rows (widened exactly); and the float64 sum of the oracle's weights within its rounding."""
+    from diffractom_b200 import _lib
+    from diffractom_b200.geometry import radon_geometry
+    nx, ny, R = 70, 40, 13
+    ang = (np.arange(R) + 0.5) * np.pi / R
+    rg = radon_geometry(ang, nx, ny, bins, width, float(bins), 0.3, 0.7, "trapezoid")
+    assert rg.n_taps == taps
+    s = torch.cuda.current_stream().cuda_stream
+    geo = torch.as_tensor(rg.geo, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(8)
+    sino = torch.randn((R, bins, ks), generator=g, device="cuda").to(torch.bfloat16).float()
+    full, fullb, row = (torch.empty((n, ks), device="cuda") for n in (nx * ny, nx * ny, nx))
+    _lib.call("dfx_radon_backward", sino.data_ptr(), full.data_ptr(), geo.data_ptr(), R, nx, ny, bins, ks, kb, 1, taps, s)
+    sb = sino.to(torch.bfloat16)
+    _lib.call("dfx_radon_backward_bf16", sb.data_ptr(), ks, fullb.data_ptr(), geo.data_ptr(), R, nx, ny, bins, ks, kb, 1,
+              taps, s)
+    assert torch.equal(full, fullb) and full.any() and not full[:, kb:].any()
+    for y in (0, 17, ny - 1):
+        pix = torch.arange(y * nx, (y + 1) * nx, dtype=torch.int32, device="cuda")
+        _lib.call("dfx_radon_backward_pixels", sino.data_ptr(), row.data_ptr(), geo.data_ptr(), R, nx, ny, bins, ks, kb, 1,
+                  taps, pix.data_ptr(), nx, s)
+        assert torch.equal(row, full[y * nx:(y + 1) * nx])
+    # float64: the trapezoid of a unit step along the axis with the larger coefficient
+    geo64 = np.asarray(rg.geo, np.float64)
+    yy, xx = (v.ravel() for v in np.mgrid[:ny, :nx])
+    want, size = np.zeros((nx * ny, kb)), np.zeros((nx * ny, kb))
+    src = sino[:, :, :kb].double().cpu().numpy()
+    for a in range(R):
+        t = geo64[a, 0] * xx + geo64[a, 1] * yy + geo64[a, 2]
+        A = max(abs(geo64[a, 0]), abs(geo64[a, 1]))
+        w = np.clip((1 + A) / 2 - np.abs(t[:, None] - np.arange(bins)), 0.0, min(1.0, A)) / A * geo64[a, 3]
+        want += w @ src[a]
+        size += w @ np.abs(src[a])
+    # the place of a pixel is rounded to 2^-24 of some hundred bins, a weight's slope is 1 / A, 5 taps of each angle
+    bound = 2 * R * taps * 2.0 ** -24 * size + 2.0 ** -24 * bins * 4 * np.abs(src).max() * R * 0.7 * taps
+    assert (np.abs(full[:, :kb].double().cpu().numpy() - want) <= bound).all()
