@@ -431,7 +431,7 @@ __global__ void __launch_bounds__(SP_ROWS) spmm_forward_b4_kernel(
 // kernel's) bit for bit.
 constexpr int ZT_G = 9;                  // 32-line groups per warp at most (288 lines)
 // entries in flight per warp for MT line groups
-constexpr int zt_uf(int mt, bool wide) { return mt <= 2 ? 8 : wide ? 3 : 4; }
+constexpr int zt_uf(int mt, bool wide) { return mt <= 2 ? (wide ? 4 : 8) : wide ? 3 : 4; }
 constexpr int zt_ua(int mt) { return mt <= 2 ? 8 : 4; }
 
 // a0 = fmaf(v, z0, a0), a1 = fmaf(v, z1, a1) in one instruction (same rounding as two fmaf)
@@ -848,17 +848,17 @@ static int launch_zt(const float *zt, const int32_t *fb_ptr, const uint16_t *fb_
     // SM as the line 270 blocks of 99 x 99 64 -> 90 us, 180 of 128 x 128 78 -> 90, 162 of 80 x 80 31 -> 25: the rows are
     // taken longest first and the write-back has whole segments.
     while (nb > 1 && cdiv(ncb, nb) * nyb * na < nsm) --nb;
-    // three blocks of 80 registers per SM with three entries in flight per warp, or two of 128 with four. From four
-    // waves of three on the former: 36 waves (360 angles at 256 x 256 pixels, 1012 channels) 1.67 against 1.87 ms, 6
-    // waves (180 at 99 x 99) 0.53 against 0.60, 4.1 waves 0.187 against 0.199. Under a wave the latter: 0.6 waves (18
-    // angles at 99 x 99) 64 against 76 us, 1.0 (45 at 128 x 128) 157 against 181. Between them the former is 5 to 19 %
-    // ahead from 1.5 waves on (36 angles at 256 x 256, 3.6 waves: 203 against 220 us; 120 at 64 x 64, 2.7: 204 against
-    // 253): there the rule is not yet at its best.
-    if constexpr (MT > 2) {
-        if (cdiv(ncb, nb) * nyb * na >= 4LL * 3 * nsm)
-            return launch_zt_as<MT, true>(zt, fb_ptr, fb_k, fb_v, fb_mask, data, omegas, r0, na, my, ly, nyb, P, C, ncb,
-                                          nb, kb, st);
-    }
+    // Three blocks of 80 registers per SM with three entries in flight per warp (four up to 64 lines), or two of 128 with
+    // four (eight): the former where it saves a wave of blocks. Blocks per SM, times of the former and the latter: 1.8
+    // (18 angles at 99 x 99 pixels) 76 and 64 us; 2.0 (30 at 64 x 64) 74 and 82; 2.7 (45 at 80 x 80) 39 and 46; 3.0 (45
+    // at 128 x 128) 181 and 158; 4.6 (45 at 99 x 99) 162 and 174; 5.5 (18 at 256 x 256, 1012 channels) 111 and 120; 8.1
+    // (120 at 64 x 64) 204 and 253; 18 (180 at 99 x 99) 530 and 596; 109 (360 at 256 x 256) 1669 and 1872. Up to 64
+    // lines: 2.8 (53 lines, 18 angles of 180 eta bins x 8 rings, 500 channels) 18.9 and 24.3, 3.7 (20 lines, 45 of 90 x
+    // 8) 47 and 39, 7.0 (33 lines, 45 of 180 x 8) 25 and 30.
+    const int64_t blocks = cdiv(ncb, nb) * nyb * na;
+    if (cdiv(blocks, 3LL * nsm) < cdiv(blocks, 2LL * nsm))
+        return launch_zt_as<MT, true>(zt, fb_ptr, fb_k, fb_v, fb_mask, data, omegas, r0, na, my, ly, nyb, P, C, ncb, nb,
+                                      kb, st);
     return launch_zt_as<MT, false>(zt, fb_ptr, fb_k, fb_v, fb_mask, data, omegas, r0, na, my, ly, nyb, P, C, ncb, nb, kb,
                                    st);
 }

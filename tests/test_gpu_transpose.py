@@ -113,9 +113,9 @@ def test_lines_fastest_products_against_float64(shift):
     assert (np.abs(adj.cpu().numpy()[:, :, :kb] - wadj) <= 24 * 2.0 ** -24 * sadj).all()
 
 
-@pytest.mark.parametrize("my", [70, 263])
+@pytest.mark.parametrize("my", [20, 53, 70, 263])
 def test_lines_fastest_forward_with_many_blocks(my):
-    """More than four waves of blocks (the variant with three blocks per SM): the channel-fastest form's bits."""
+    """Many blocks (the variants with three of them per SM): the channel-fastest form's bits."""
     from diffractom_b200 import _lib
     rng = np.random.default_rng(7)
     P, C, R, kb, ks = 8, 36, 400, 40, 40               # 400 angles x 5 blocks of two eta blocks
